@@ -61,10 +61,7 @@ __device__ __forceinline__ void cell_xyz(const DevState<real> &s, int c, int &cx
 // Pass 1: wrap (Domain::fix_position: one if / else-if per periodic axis),
 // cell index, copy the atom to the temporaries, count atoms per cell.
 template <typename real>
-__global__ void k_bin_count(DevState<real> s) {
-  if (*s.flag == 0) return;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= s.n) return;
+__device__ __forceinline__ void bin_atom(const DevState<real> &s, int i) {
   double p[3] = {s.x[i], s.y[i], s.z[i]};
   int c[3];
   bool clamped = false;
@@ -96,6 +93,12 @@ __global__ void k_bin_count(DevState<real> s) {
   s.tmol[i] = s.mol[i];
   s.tcell[i] = cell;
   atomicAdd(&s.cell_count[cell], 1);
+}
+template <typename real>
+__global__ void k_bin_count(DevState<real> s) {
+  if (*s.flag == 0) return;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < s.n) bin_atom(s, i);
 }
 
 // Exclusive scan of cell_count into cell_start, in three passes over blocks
@@ -169,42 +172,42 @@ __global__ void __launch_bounds__(1024) k_scan_add(const int *__restrict__ flag,
 // fixed by k_rank below, so the atomics here do not make the result depend
 // on scheduling).
 template <typename real>
-__global__ void k_bin_scatter(DevState<real> s) {
-  if (*s.flag == 0) return;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= s.n) return;
+__device__ __forceinline__ void scatter_atom(const DevState<real> &s, int i) {
   const int c = s.tcell[i];
   const int slot = s.cell_start[c] + atomicAdd(&s.cell_fill[c], 1);
   s.slot_atom[slot] = i;
 }
+template <typename real>
+__global__ void k_bin_scatter(DevState<real> s) {
+  if (*s.flag == 0) return;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < s.n) scatter_atom(s, i);
+}
 
 // Pass 3: inside each cell, order atoms by id (deterministic layout).
+// Atom i's place in cell order.
+template <typename real>
+__device__ __forceinline__ int place_of(const DevState<real> &s, int i) {
+  const int c = s.tcell[i];
+  const int b = s.cell_start[c], e = s.cell_start[c + 1];
+  const int key = s.tid[i];
+  int rank = 0;
+  for (int u = b; u < e; ++u) rank += (s.tid[s.slot_atom[u]] < key) ? 1 : 0;
+  return b + rank;
+}
 template <typename real>
 __global__ void k_rank(DevState<real> s) {
   if (*s.flag == 0) return;
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= s.n) return;
   const int i = s.slot_atom[t];
-  const int c = s.tcell[i];
-  const int b = s.cell_start[c], e = s.cell_start[c + 1];
-  const int key = s.tid[i];
-  int rank = 0;
-  for (int u = b; u < e; ++u) rank += (s.tid[s.slot_atom[u]] < key) ? 1 : 0;
-  s.perm[b + rank] = i;
+  s.perm[place_of(s, i)] = i;
 }
 
 // Pass 4: gather into cell order, build the cell-local coordinates and the
 // ghost-zone classification, and clear the per-cell counters for next time.
 template <typename real>
-__global__ void k_permute(DevState<real> s) {
-  if (*s.flag == 0) return;
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k < s.cells.ncells) {
-    s.cell_count[k] = 0;
-    s.cell_fill[k] = 0;
-  }
-  if (k >= s.n) return;
-  const int i = s.perm[k];
+__device__ __forceinline__ void place_atom(const DevState<real> &s, int k, int i, typename V4<real>::t *x4) {
   const double p[3] = {s.tx[i], s.ty[i], s.tz[i]};
   s.x[k] = p[0];
   s.y[k] = p[1];
@@ -243,10 +246,20 @@ __global__ void k_permute(DevState<real> s) {
   } else {
     q.w = (double)ty;
   }
-  s.x4[k] = q;
+  x4[k] = q;
   s.xb[k] = make_float4((float)(p[0] - s.box.ctr[0]), (float)(p[1] - s.box.ctr[1]), (float)(p[2] - s.box.ctr[2]),
                         __int_as_float(cc[0]));
   s.gcls[k] = (int8_t)code;
+}
+template <typename real>
+__global__ void k_permute(DevState<real> s) {
+  if (*s.flag == 0) return;
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k < s.cells.ncells) {
+    s.cell_count[k] = 0;
+    s.cell_fill[k] = 0;
+  }
+  if (k < s.n) place_atom(s, k, s.perm[k], s.x4);
 }
 
 // |pa - image(pb, shift)|^2 < rl^2 in the reference's FP64 order:
@@ -315,19 +328,24 @@ __device__ __forceinline__ size_t list_slot(int cnt, int log2_tpa, size_t stride
 }
 
 
+// The live pieces of one warp's stencil rows (list_search_warp): where each
+// starts in the sequence of candidates (one more than the pieces), its image
+// offset and first candidate, its entry bits; 2 S^2 pieces at most.
+constexpr int PIECES_MAX = 2 * (2 * STENCIL_R_MAX + 1) * (2 * STENCIL_R_MAX + 1);
+struct WarpPieces {
+  int *off;
+  float4 *geo;  // image offset bx, by, bz; first candidate (int bits)
+  uint32_t *pc;
+};
+
 // The same search with one WARP per atom, for systems too small to fill the
 // GPU with one thread per atom: the 32 lanes take consecutive candidates of a
 // stencil cell, and a ballot keeps the accepted ones in candidate order, so
-// the list is identical to the one-thread-per-atom build.  Launched with 128
-// threads (four warps: the per-warp piece tables); a register cap rather than
-// launch bounds keeps the sweep free of spills.
+// the list is identical to the one-thread-per-atom build.  Returns the
+// number of neighbours found.
 template <typename real>
-__global__ void __maxnreg__(80) k_build_list_warp(DevState<real> s, int count_only, int log2_tpa) {
-  if (*s.flag == 0) return;
-  if (blockIdx.x == 0 && threadIdx.x == 0 && !count_only) atomicAdd(s.n_builds, 1);
-  const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (i >= s.n) return;  // whole warp leaves together
+__device__ __forceinline__ int list_search_warp(const DevState<real> &s, int i, int lane, const WarpPieces &wp,
+                                                 int count_only, int log2_tpa) {
   int cx, cy, cz;
   cell_xyz(s, s.cell[i], cx, cy, cz);
   const float4 xi = s.xb[i];
@@ -340,14 +358,17 @@ __global__ void __maxnreg__(80) k_build_list_warp(DevState<real> s, int count_on
   const unsigned lt = (1u << lane) - 1u;
   int cnt = 0;
   if (nc0 >= S) {
-    // Row mode: the stencil's S*S rows (dz, dy), each at most three
-    // contiguous atom ranges (the sx = -1, 0, +1 pieces of the unwrapped x
-    // range [cx-R, cx+R]).  The lanes first load every piece's range in one
-    // parallel round trip, then the warp sweeps the pieces in stencil order,
-    // 32 candidates at a time (the same entries, in the same order, as the
-    // cell-by-cell sweep below).
-    constexpr int KP = (3 * (2 * MAX_STENCIL_R + 1) * (2 * MAX_STENCIL_R + 1) + 31) / 32;
-    const int P = 3 * S * S;
+    // Row mode: the stencil's S*S rows (dz, dy), one per lane.  A row's
+    // unwrapped x range [cx-R, cx+R] is at most two contiguous atom ranges
+    // (pieces): with nc0 >= S it crosses one end of the box at most.  The
+    // lanes first load every piece's range in one parallel round trip, then
+    // the warp sweeps the pieces in stencil order, 32 candidates at a time
+    // (the same entries, in the same order, as the cell-by-cell sweep below).
+    // One lane per piece, three per row, took two more rounds and scans per
+    // atom: 97 -> 67 us per rebuild of 32,001 LJ atoms inside k_steps (search
+    // and pair force), 37.6 -> 35.2 us per step with one kernel per stage.
+    constexpr int KR = ((2 * STENCIL_R_MAX + 1) * (2 * STENCIL_R_MAX + 1) + 31) / 32;  // rounds over the rows
+    const int rows = S * S;
     // Each row is clipped to the cells that meet the rl sphere around atom i:
     // with g_y, g_z the atom's distances to the row's y and z slabs, only
     // cells within h = sqrt(rl^2 - g_y^2 - g_z^2) of it in x can hold a
@@ -367,23 +388,27 @@ __global__ void __maxnreg__(80) k_build_list_warp(DevState<real> s, int count_on
     const float dlt = 1e-3f * fminf(wx, fminf(wy, wz));
     const float rc2 = s.rl_sq_hi;
     const bool clip = *s.clamp_mark != *s.build_epoch;
-    // per piece: first candidate, length, and the list-entry bits of the
+    // Per piece: first candidate, length, and the list-entry bits of the
     // piece (dy, dz fields and cell_x(j) + dxc + R in the dx field, less
     // cell_x(j); wrapping 32-bit arithmetic, exact once cell_x(j) is added)
     // with the image shift (sx + 1) | (sy + 1) << 2 | (sz + 1) << 4 in the
-    // low bits (the j field, zero in the entry bits)
-    int pst[KP], plen[KP];
-    uint32_t pcode[KP];
+    // low bits (the j field, zero in the entry bits).  The live pieces, in
+    // stencil order, laid end to end: a per-warp table in shared memory of
+    // each piece's start in that sequence, first candidate, image offset and
+    // entry bits.  The warp then sweeps the sequence 32 candidates at a time,
+    // so a round spans piece boundaries instead of idling the lanes past the
+    // end of a short row.
+    constexpr uint32_t kUnshifted = 1u | (1u << 2) | (1u << 4);
+    int nlive = 0, total = 0;
 #pragma unroll
-    for (int k = 0; k < KP; ++k) {
-      const int p = 32 * k + lane;
-      pst[k] = 0;
-      plen[k] = 0;
-      pcode[k] = 0;
-      if (p < P) {
-        const int r = p / 3, sx = p % 3 - 1;
-        const int dz = r / S - R, dy = r % S - R;
-        const int sz = floor_div(cz + dz, nc2), sy = floor_div(cy + dy, nc1);
+    for (int k = 0; k < KR; ++k) {
+      const int r = 32 * k + lane;
+      int pst[2] = {0, 0}, plen[2] = {0, 0}, psx[2] = {0, 0}, dy = 0, dz = 0, sy = 0, sz = 0;
+      if (r < rows) {
+        dz = r / S - R;
+        dy = r % S - R;
+        sz = floor_div(cz + dz, nc2);
+        sy = floor_div(cy + dy, nc1);
         const float gy = fmaxf(fmaxf(dy * wy - fy, fy - (dy + 1) * wy) - dlt, 0.f);
         const float gz = fmaxf(fmaxf(dz * wz - fz, fz - (dz + 1) * wz) - dlt, 0.f);
         const float h2 = rc2 - gy * gy - gz * gz;
@@ -396,58 +421,49 @@ __global__ void __maxnreg__(80) k_build_list_warp(DevState<real> s, int count_on
           ua = cx + max(-R, min(R + 1, __float2int_rd((fx - hx) * ivx)));
           ub = cx + min(R, max(-R - 1, __float2int_rd((fx + hx) * ivx)));
         }
-        if (sx < 0) ub = min(ub, -1);
-        if (sx == 0) {
-          ua = max(ua, 0);
-          ub = min(ub, nc0 - 1);
-        }
-        if (sx > 0) ua = max(ua, nc0);
-        const bool live = ua <= ub && (sz == 0 || s.box.bc[2]) && (sy == 0 || s.box.bc[1]) && (sx == 0 || s.box.bc[0]);
-        if (live) {
+        if (ua <= ub && (sz == 0 || s.box.bc[2]) && (sy == 0 || s.box.bc[1])) {
+          // the range split where it leaves the box: u < split, u >= split
+          const int split = ua < 0 ? 0 : nc0;
+          psx[0] = ua < 0 ? -1 : (ua >= nc0 ? 1 : 0);
+          psx[1] = ua < 0 ? 0 : 1;
           const int rowbase = nc0 * (cy + dy - sy * nc1 + nc1 * (cz + dz - sz * nc2));
-          pst[k] = s.cell_start[rowbase + ua - sx * nc0];
-          plen[k] = s.cell_start[rowbase + ub - sx * nc0 + 1] - pst[k];
-          const int dxc = sx * nc0 - cx;  // dx = cell_x(j) + dxc
-          pcode[k] = (list_entry(0, 0, dy, dz, R, S) + (uint32_t)dxc * (1u << CODE_SHIFT)) |
-                     (uint32_t)((sx + 1) | ((sy + 1) << 2) | ((sz + 1) << 4));
+          const int b0 = ua >= nc0 ? ub : min(ub, split - 1);
+          if (psx[0] == 0 || s.box.bc[0]) {
+            pst[0] = s.cell_start[rowbase + ua - psx[0] * nc0];
+            plen[0] = s.cell_start[rowbase + b0 - psx[0] * nc0 + 1] - pst[0];
+          }
+          if (ua < split && ub >= split && (psx[1] == 0 || s.box.bc[0])) {
+            pst[1] = s.cell_start[rowbase + split - psx[1] * nc0];
+            plen[1] = s.cell_start[rowbase + ub - psx[1] * nc0 + 1] - pst[1];
+          }
         }
       }
-    }
-    // The live pieces, in stencil order, laid end to end: a per-warp table
-    // in shared memory of each piece's start in that sequence, first
-    // candidate, image offset and entry bits.  The warp then sweeps the
-    // sequence 32 candidates at a time, so a round spans piece boundaries
-    // instead of idling the lanes past the end of a short row.
-    constexpr uint32_t kUnshifted = 1u | (1u << 2) | (1u << 4);
-    constexpr int PMAX = 3 * (2 * MAX_STENCIL_R + 1) * (2 * MAX_STENCIL_R + 1);
-    __shared__ int s_off[4][PMAX + 1];
-    __shared__ float4 s_geo[4][PMAX];  // image offset bx, by, bz; first candidate (int bits)
-    __shared__ uint32_t s_pc[4][PMAX];
-    const int w = threadIdx.x >> 5;
-    int nlive = 0, total = 0;
-#pragma unroll
-    for (int k = 0; k < KP; ++k) {
-      const int len = plen[k];
+      const int len = plen[0] + plen[1];
       int incl = len;  // inclusive scan of the lengths across the lanes
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
         const int y = __shfl_up_sync(0xffffffffu, incl, o);
         if (lane >= o) incl += y;
       }
-      const unsigned live = __ballot_sync(0xffffffffu, len > 0);
-      if (len > 0) {
-        const int q = nlive + __popc(live & lt);
-        const uint32_t code = pcode[k] & 63u;
-        const int sx = (int)(code & 3u) - 1, sy = (int)((code >> 2) & 3u) - 1, sz = (int)(code >> 4) - 1;
-        s_off[w][q] = total + incl - len;
-        s_geo[w][q] = make_float4(sx * s.box.Lf[0] - xi.x, sy * s.box.Lf[1] - xi.y, sz * s.box.Lf[2] - xi.z,
-                                  __int_as_float(pst[k]));
-        s_pc[w][q] = pcode[k];
+      const unsigned live0 = __ballot_sync(0xffffffffu, plen[0] > 0), live1 = __ballot_sync(0xffffffffu, plen[1] > 0);
+      int q = nlive + __popc(live0 & lt) + __popc(live1 & lt), at = total + incl - len;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        if (plen[h] > 0) {
+          const int sx = psx[h], dxc = sx * nc0 - cx;  // dx = cell_x(j) + dxc
+          wp.off[q] = at;
+          wp.geo[q] = make_float4(sx * s.box.Lf[0] - xi.x, sy * s.box.Lf[1] - xi.y, sz * s.box.Lf[2] - xi.z,
+                                  __int_as_float(pst[h]));
+          wp.pc[q] = (list_entry(0, 0, dy, dz, R, S) + (uint32_t)dxc * (1u << CODE_SHIFT)) |
+                     (uint32_t)((sx + 1) | ((sy + 1) << 2) | ((sz + 1) << 4));
+          at += plen[h];
+          ++q;
+        }
       }
-      nlive += __popc(live);
+      nlive += __popc(live0) + __popc(live1);
       total += __shfl_sync(0xffffffffu, incl, 31);
     }
-    if (lane == 0) s_off[w][nlive] = total;
+    if (lane == 0) wp.off[nlive] = total;
     __syncwarp();
     int q0 = 0;  // the live piece that holds candidate `base`
     for (int base = 0; base < total; base += 32) {
@@ -455,7 +471,7 @@ __global__ void __maxnreg__(80) k_build_list_warp(DevState<real> s, int count_on
       const int qt = q0 + 1 + lane;
       unsigned bit = 0u;
       if (qt < nlive) {
-        const int o = s_off[w][qt];
+        const int o = wp.off[qt];
         if (o < base + 32) bit = 1u << (o - base);
       }
       const unsigned starts = __reduce_or_sync(0xffffffffu, bit);
@@ -466,9 +482,9 @@ __global__ void __maxnreg__(80) k_build_list_warp(DevState<real> s, int count_on
       uint32_t pc = 0;
       if (c < total) {
         const int qp = q0 + __popc(starts & ((2u << lane) - 1u));  // this lane's piece
-        const float4 g = s_geo[w][qp];
-        pc = s_pc[w][qp];
-        j = __float_as_int(g.w) + (c - s_off[w][qp]);
+        const float4 g = wp.geo[qp];
+        pc = wp.pc[qp];
+        j = __float_as_int(g.w) + (c - wp.off[qp]);
         const uint32_t code = pc & 63u;
         const bool shifted = code != kUnshifted;
         if (!shifted ? j != i : true) {
@@ -491,7 +507,7 @@ __global__ void __maxnreg__(80) k_build_list_warp(DevState<real> s, int count_on
       }
       cnt += __popc(m);
       q0 += __popc(starts);  // the piece that holds candidate base + 32
-      if (q0 + 1 < nlive && s_off[w][q0 + 1] <= base + 32) ++q0;
+      if (q0 + 1 < nlive && wp.off[q0 + 1] <= base + 32) ++q0;
     }
   } else
   for (int dz = -R; dz <= R; ++dz) {
@@ -538,6 +554,21 @@ __global__ void __maxnreg__(80) k_build_list_warp(DevState<real> s, int count_on
     if (!count_only && cnt > s.cap) atomicOr(s.err, ERR_OVERFLOW);
     atomicMax(s.max_count, cnt);
   }
+  return cnt;
+}
+
+// Launched with 128 threads (four warps: the per-warp piece tables); a
+// register cap rather than launch bounds keeps the sweep free of spills.
+template <typename real>
+__global__ void __maxnreg__(80) k_build_list_warp(DevState<real> s, int count_only, int log2_tpa) {
+  if (*s.flag == 0) return;
+  if (blockIdx.x == 0 && threadIdx.x == 0 && !count_only) atomicAdd(s.n_builds, 1);
+  __shared__ int off[4][PIECES_MAX + 1];
+  __shared__ float4 geo[4][PIECES_MAX];
+  __shared__ uint32_t pc[4][PIECES_MAX];
+  const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, w = threadIdx.x >> 5;
+  if (i >= s.n) return;  // whole warp leaves together
+  list_search_warp(s, i, threadIdx.x & 31, WarpPieces{off[w], geo[w], pc[w]}, count_only, log2_tpa);
 }
 
 // Pass 5: the pair search, one thread per atom over the (2R+1)^3 stencil.

@@ -20,10 +20,18 @@
 
 namespace cvr {
 
-enum : int { ERR_NAN = 1, ERR_OVERFLOW = 2, ERR_GEOMETRY = 4, ERR_KSPACE_TC = 8 };
+enum : int { ERR_NAN = 1, ERR_OVERFLOW = 2, ERR_GEOMETRY = 4, ERR_KSPACE_TC = 8, ERR_BARRIER = 16 };
 constexpr int CODE_SHIFT = 23;  // first of the three 3-bit stencil-offset fields
 constexpr unsigned INDEX_MASK = (1u << CODE_SHIFT) - 1u;
 constexpr int MAX_STENCIL_R = 3;  // dx + R must fit in 3 bits
+// Stencil radius in cells: cells are at least rl / R wide, so every pair
+// within rl is at most R cells apart on each axis (R = 1 was measured: the
+// pair kernel gathers better, the list search costs more, the step is slower).
+#ifndef CVR_STENCIL_R
+#define CVR_STENCIL_R 2
+#endif
+constexpr int STENCIL_R_MAX = CVR_STENCIL_R;
+static_assert(STENCIL_R_MAX <= MAX_STENCIL_R, "stencil offsets must fit the list entry");
 constexpr int MAX_TYPES = 16;
 constexpr int MAX_KMAX = 31;
 
