@@ -22,13 +22,7 @@
 #include "cvr_device.cuh"
 #include "cvr_force.cuh"
 #include "cvr_kforce_tc.cuh"
-
-// Stencil radius in cells: cells are at least rl / R wide, so every pair
-// within rl is at most R cells apart on each axis (R = 1 was measured: the
-// pair kernel gathers better, the list search costs more, the step is slower).
-#ifndef CVR_STENCIL_R
-#define CVR_STENCIL_R 2
-#endif
+#include "cvr_steps.cuh"
 
 using namespace cvr;
 
@@ -48,6 +42,10 @@ constexpr int KMZ = 16;    // k-force: Z[m] held in registers up to this many m-
 #endif
 constexpr int KF_WMAX = CVR_KF_WMAX;  // k-force: most warps per block of 32 atoms
 constexpr int KRW = 16;    // warps of the S(k) chunk reduction
+// Many steps in one launch (k_steps) up to this many atoms, the range of the
+// warp-per-atom list search (per step, one kernel per stage -> k_steps: 20.5 ->
+// 7.0 us at 500 LJ atoms, 50.1 -> 40.7 at 65,001).
+constexpr int64_t STEPS_MAX_ATOMS = 65536;
 constexpr size_t KF_COEF_SMEM = 72 * 1024;  // k-force: shared memory for staged column coefficients
 
 struct DBuf {
@@ -193,6 +191,14 @@ struct cvr_ctx {
   int64_t graph_kernels[2] = {0, 0};
   long long *counters{};
   long long counter_src[2] = {0, 0};
+  // many steps in one launch (k_steps): second pair-coordinate buffer,
+  // control words, thermostat sums, thermo-record sums, positions at the
+  // build, launch parity
+  int sms = 148;
+  void *x4b{};
+  unsigned long long *step_ctrl{};
+  double *step_part{}, *step_rec{}, *step_pos{};
+  int step_launch = 0;
   // Langevin integrator (md_simulator.cpp:670-811)
   int integrator = 0;  // 0 velocity Verlet, 1 velocity Verlet Langevin
   double lgv_temperature = -1, lgv_friction = 0, lgv_kb = -1, lgv_kbt = -1;
@@ -615,6 +621,10 @@ int alloc_atoms(cvr_ctx *c, int64_t n) {
   if ((r = dalloc(c, (unsigned char **)&c->ay, n * rs))) return r;
   if ((r = dalloc(c, (unsigned char **)&c->az, n * rs))) return r;
   if ((r = dalloc(c, (unsigned char **)&c->x4, n * 4 * rs))) return r;
+  const size_t ns = n <= STEPS_MAX_ATOMS ? n : 0;  // the buffers of k_steps
+  if ((r = dalloc(c, (unsigned char **)&c->x4b, ns * 4 * rs))) return r;
+  if ((r = dalloc(c, &c->step_rec, 2 * steps_record_doubles(ns)))) return r;
+  if ((r = dalloc(c, &c->step_pos, 3 * ns))) return r;
   // per-atom arrays that a replay after a list overflow restores
   c->snap_pairs.clear();
   c->snap_bytes.clear();
@@ -661,7 +671,7 @@ int alloc_list(cvr_ctx *c, int cap) {
 // 34.2 vs thread 38.5 us at 32,000 atoms, 59.5 vs 50.7 us at 108,000).
 int list_kernel_kind(const cvr_ctx *c) {
   if (c->list_kernel != CVR_LIST_AUTO) return c->list_kernel;
-  return (c->n <= 65536) ? CVR_LIST_WARP : CVR_LIST_THREAD;
+  return (c->n <= STEPS_MAX_ATOMS) ? CVR_LIST_WARP : CVR_LIST_THREAD;
 }
 
 bool phase_in_drift(const cvr_ctx *c);
@@ -938,8 +948,7 @@ void set_smem_attrs(cvr_ctx *c) {
   KForceTable<real, KMZ>::attrs(c);
 }
 
-template <typename real>
-void launch_thermo(cvr_ctx *c, double *out) {
+ThermoArgs thermo_args(cvr_ctx *c, double *out) {
   ThermoArgs t{};
   t.ke_part = c->ke_part;
   t.n_ke = c->n_ke_blocks;
@@ -965,7 +974,11 @@ void launch_thermo(cvr_ctx *c, double *out) {
   t.n_builds = c->flags + 3;
   t.counters = c->counters;
   t.out = out;
-  k_thermo<<<1, THERMO_THREADS, 0, c->stream>>>(t);
+  return t;
+}
+
+void launch_thermo(cvr_ctx *c, double *out) {
+  k_thermo<<<1, THERMO_THREADS, 0, c->stream>>>(thermo_args(c, out));
   c->launches++;
 }
 
@@ -1171,6 +1184,21 @@ LangevinArgs langevin_args(cvr_ctx *c) {
   return lg;
 }
 
+ThermostatArgs thermostat_args(cvr_ctx *c) {
+  ThermostatArgs t = c->tstat;
+  const int bcsum = c->bc[0] + c->bc[1] + c->bc[2];
+  const int n_r_df = (bcsum == 0) ? 6 : (bcsum == 3 ? 3 : 6 - bcsum);  // atom_data.cpp:322-349
+  t.com_removed = (n_r_df >= 1 && n_r_df <= 3) ? 1 : 0;
+  t.dof = 3.0 * (double)c->n - n_r_df;
+  t.total_mass = c->total_mass;
+  t.k_b = c->k_b;
+  t.ke_part = c->ke_part;
+  t.n_ke = c->n_ke_blocks;
+  t.counters = c->counters;
+  t.scal = c->d_tscal;
+  return t;
+}
+
 // deferred: the step's kick is left to the next step's k_kick_drift (only
 // where defer_kick allows it, never with a thermo record).
 template <typename real>
@@ -1193,17 +1221,7 @@ int launch_step_tail(cvr_ctx *c, bool th, bool deferred = false) {
       k_kick<real, false><<<nb, 256, 0, c->stream>>>(s, c->dt, c->ke_part, c->counters);
     }
     if (c->tstat.kind && c->integrator == 0) {
-      ThermostatArgs t = c->tstat;
-      const int bcsum = c->bc[0] + c->bc[1] + c->bc[2];
-      const int n_r_df = (bcsum == 0) ? 6 : (bcsum == 3 ? 3 : 6 - bcsum);  // atom_data.cpp:322-349
-      t.com_removed = (n_r_df >= 1 && n_r_df <= 3) ? 1 : 0;
-      t.dof = 3.0 * (double)c->n - n_r_df;
-      t.total_mass = c->total_mass;
-      t.k_b = c->k_b;
-      t.ke_part = c->ke_part;
-      t.n_ke = c->n_ke_blocks;
-      t.counters = c->counters;
-      t.scal = c->d_tscal;
+      const ThermostatArgs t = thermostat_args(c);
       k_thermostat_coef<<<1, 256, 0, c->stream>>>(t);
       if (th)
         k_thermostat_apply<real, true><<<nb, 256, 0, c->stream>>>(s, t.kind, c->d_tscal, c->ke_part);
@@ -1213,7 +1231,7 @@ int launch_step_tail(cvr_ctx *c, bool th, bool deferred = false) {
     }
     c->launches++;
   }
-  if (th) launch_thermo<real>(c, c->d_thermo);
+  if (th) launch_thermo(c, c->d_thermo);
   return CVR_OK;
 }
 
@@ -1251,6 +1269,75 @@ int stage_reference_eta(cvr_ctx *c, int slot) {
   CVR_CUDA(c, cudaMemcpyAsync(c->d_eta, h, 3 * (size_t)n * sizeof(double), cudaMemcpyHostToDevice, c->stream));
   CVR_CUDA(c, cudaEventRecord(c->eta_done[slot], c->stream));
   return CVR_OK;
+}
+
+// Whether a run's steps go through k_steps: LJ only (the k-space
+// chain, the Langevin noise and the debug modes keep one kernel per stage)
+// and a system whose list is searched by a warp per atom.
+bool steps_in_one(const cvr_ctx *c) {
+  return c->use_graphs && !c->timing && c->lj_on && !c->ewr_on && !(c->ewk_on && c->nk > 0) && !c->all_atom &&
+         c->integrator == 0 && !c->sc_on && !(c->ewk_on && c->dipole_mode) && c->n <= STEPS_MAX_ATOMS &&
+         (c->tpa == 32 || c->tpa == 8) && list_kernel_kind(c) == CVR_LIST_WARP;
+}
+
+template <typename real, int TPA, bool ONE_TYPE, bool FIXED>
+int launch_steps_t(cvr_ctx *c, int nsteps, int64_t every, int64_t done) {
+  // every SM (one block each at most: its co-residence is what the barriers
+  // need) down to four warps per block, one per scheduler: a small system's
+  // stages are latency chains, which share nothing on an SM of their own
+  const int groups = grid_for(c->n, 32 / TPA);
+  const int grid = std::min(c->sms, grid_for(groups, 4));
+  const int threads = std::min(STEP_THREADS, 32 * grid_for(groups, grid));
+  const double h = FIXED ? c->L[0] / std::ldexp(1.0, 32) : 1.0;  // as launch_pair_t
+  StepArgs<real> a{};
+  a.coef = (const PairCoef<real> *)c->d_coef;
+  a.fscale = (real)(1.0 / h);
+  a.ignore_intra = c->ignore_intra;
+  a.use_mol = c->use_mol ? 1 : 0;
+  a.log2_tpa = c->log2_tpa;
+  a.dt = c->dt;
+  a.nsteps = nsteps;
+  a.x4b = (typename V4<real>::t *)c->x4b;
+  a.bx = c->step_pos;
+  a.by = a.bx + c->n;
+  a.bz = a.by + c->n;
+  a.ctrl = c->step_ctrl;
+  a.launch = c->step_launch;
+  c->step_launch ^= 1;
+  a.counters = c->counters;
+  a.ts = thermostat_args(c);
+  a.part = c->step_part;
+  for (int q = 0; q < 2; ++q) {
+    a.ev_warp[q] = c->step_rec + q * steps_record_doubles(c->n);
+    a.ke_warp[q] = a.ev_warp[q] + 3 * c->n;
+  }
+  a.every = (int)std::min<int64_t>(every, INT32_MAX);
+  a.done = every > 0 ? (int)(done % every) : 0;
+  if (every > 0) a.th = thermo_args(c, c->d_thermo);
+  DevState<real> s = dev_state<real>(c);
+  const size_t smem = steps_smem(threads / 32);
+  auto kernel = k_steps<real, TPA, ONE_TYPE, FIXED>;
+  CVR_CUDA(c, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  void *args[] = {&s, &a};
+  CVR_CUDA(c, cudaLaunchCooperativeKernel((const void *)kernel, dim3(grid), dim3(threads), args, smem, c->stream));
+  c->launches++;
+  return CVR_OK;
+}
+
+template <typename real, bool FIXED>
+int launch_steps_f(cvr_ctx *c, int nsteps, int64_t every, int64_t done) {
+  const bool one = c->n_types == 1 && !c->use_mol && !(c->jump_tol > 0);
+  if (c->tpa == 32)
+    return one ? launch_steps_t<real, 32, true, FIXED>(c, nsteps, every, done) : launch_steps_t<real, 32, false, FIXED>(c, nsteps, every, done);
+  return one ? launch_steps_t<real, 8, true, FIXED>(c, nsteps, every, done) : launch_steps_t<real, 8, false, FIXED>(c, nsteps, every, done);
+}
+
+template <typename real>
+int launch_steps(cvr_ctx *c, int nsteps, int64_t every, int64_t done) {
+  if constexpr (sizeof(real) == 4) {
+    if (c->fixed) return launch_steps_f<real, true>(c, nsteps, every, done);
+  }
+  return launch_steps_f<real, false>(c, nsteps, every, done);
 }
 
 void destroy_graphs(cvr_ctx *c) {
@@ -1370,13 +1457,16 @@ int run_impl(cvr_ctx *c, int64_t nsteps, int64_t every, double *thermo) {
         c->ndist[a] = nd0[a];
       }
     }
+    const bool in_one = graphs && steps_in_one(c);
     const bool dk = defer_kick(c);
-    if (graphs && (c->graph_epoch != c->epoch || (dk && !c->g_step[1][0])))
+    if (graphs && !in_one && (c->graph_epoch != c->epoch || (dk && !c->g_step[1][0])))
       if (int r = build_graphs<real>(c)) return r;
     const int64_t launches0 = c->launches;
     bool pending = false;  // the previous step deferred its second half kick
     int64_t n_kick = 0;    // steps ending with a plain (no thermo) kick
-    for (int64_t k = 0; k < nsteps; ++k) {
+    for (int64_t k = 0; in_one && k < nsteps; k += STEPS_MAX)
+      if (int r = launch_steps<real>(c, (int)std::min<int64_t>(nsteps - k, STEPS_MAX), every, k)) return r;
+    for (int64_t k = in_one ? nsteps : 0; k < nsteps; ++k) {
       const bool th = every > 0 && ((k + 1) % every == 0);
       const int tail = th ? 2 : ((dk && k + 1 < nsteps) ? 0 : 1);
       n_kick += tail == 1;
@@ -1394,7 +1484,7 @@ int run_impl(cvr_ctx *c, int64_t nsteps, int64_t every, double *thermo) {
     int f[4];
     if (int r = read_flags(c, f)) return r;
     collect_timing(c);
-    if (graphs) {
+    if (graphs && !in_one) {
       // kernel nodes executed: per step kick_drift + condition + forces +
       // kick (fused into the k-space force, or deferred to the next step's
       // kick_drift, on plain steps when possible) + thermo record; 8 per
@@ -1405,6 +1495,10 @@ int run_impl(cvr_ctx *c, int64_t nsteps, int64_t every, double *thermo) {
       const int kick_plain = kick_in_kforce(c, false) ? 0 : 1;
       c->launches = launches0 + nsteps * (2 + tail) + n_kick * kick_plain + nrec * 2 +
                     (8 + (phase_in_drift(c) ? 1 : 0)) * (int64_t)(f[3] - f0[3]);
+    }
+    if (f[1] & ERR_BARRIER) {
+      cudaMemsetAsync(c->step_ctrl, 0, SC_WORDS * sizeof(unsigned long long), c->stream);
+      return fail(c, CVR_ERR_CUDA, "a grid barrier's wait ran out");
     }
     if (f[1] & ERR_NAN) return fail(c, CVR_ERR_NAN, "NaN acceleration");
     if (f[1] & ERR_KSPACE_TC) return fail(c, CVR_ERR_CUDA, "tensor-core k-space force: a wait ran out");
@@ -1452,7 +1546,7 @@ int compute_impl(cvr_ctx *c, double *acc, double *thermo) {
   c->counter_src[0] = c->step;
   c->counter_src[1] = 0;
   CVR_CUDA(c, cudaMemcpyAsync(c->counters, c->counter_src, sizeof(c->counter_src), cudaMemcpyHostToDevice, c->stream));
-  launch_thermo<real>(c, c->d_thermo);
+  launch_thermo(c, c->d_thermo);
   CVR_CUDA(c, cudaMemcpyAsync(c->last_thermo, c->d_thermo, CVR_N_THERMO * sizeof(double), cudaMemcpyDeviceToHost,
                               c->stream));
   if (acc) {
@@ -1479,7 +1573,11 @@ int compute_impl(cvr_ctx *c, double *acc, double *thermo) {
 // ------------------------------------------------------------------ C ABI
 namespace {
 
-int choose_tpa(int64_t n) {
+int choose_tpa(const cvr_ctx *c, int64_t n) {
+  // many steps in one launch (k_steps): one atom per warp while every warp of
+  // the grid has at most one, else four (16,001 LJ atoms: 24.9 -> 15.1 us per
+  // step mixed, 30.5 -> 18.7 FP64)
+  if (!c->ewr_on && !c->ewk_on && c->integrator == 0 && n <= STEPS_MAX_ATOMS) return n <= STEP_THREADS / 32 * c->sms ? 32 : 8;
   // enough lanes to fill 148 SMs (about 6e5 threads) without starving lanes
   if (n * 32 <= 600000) return 32;
   if (n * 8 <= 600000) return 8;
@@ -1666,7 +1764,9 @@ int cvr_create(cvr_ctx **out, const double lo[3], const double hi[3], const int 
     delete c;
     return CVR_ERR_CUDA;
   }
+  cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, device);
   if (dalloc(c, &c->flags, 6) != CVR_OK || dalloc(c, &c->counters, 2) != CVR_OK ||
+      dalloc(c, &c->step_ctrl, SC_WORDS) != CVR_OK || dalloc(c, &c->step_part, 4 * (size_t)c->sms) != CVR_OK ||
       dalloc(c, &c->d_type_hist, MAX_TYPES + 1) != CVR_OK) {
     cudaEventDestroy(c->k_fork);
     cudaEventDestroy(c->k_join);
@@ -1954,7 +2054,7 @@ int cvr_set_state(cvr_ctx *c, int64_t n, const double *pos, const double *vel, c
     if (int r = alloc_atoms(c, n)) return r;
     if (int r = dalloc(c, &c->stage, 9 * (size_t)n)) return r;
     c->cap = 0;
-    c->tpa = choose_tpa(n);
+    c->tpa = choose_tpa(c, n);
     // list interleave: TPA lanes per atom, or quads of four entries when one lane per atom
     c->log2_tpa = (c->tpa == 32) ? 5 : (c->tpa == 8 ? 3 : 2);
   }

@@ -214,6 +214,112 @@ __device__ __forceinline__ void pair_disp(const real4 &xj, const real4 &xi, uint
   }
 }
 
+// The sum over atom i's list row, this lane's share (lane of TPA; the lanes'
+// shares are added by the caller), and the atom's type.
+template <typename real, int TPA, bool LJ, bool EWR, bool EV, bool ONE_TYPE, bool FIXED>
+__device__ __forceinline__ void pair_row(PairAcc<real> &A, int &ti, const DevState<real> &s,
+                                         const typename V4<real>::t *x4, int i, int lane, const PairCoef<real> *coef,
+                                         const Stencil<real> &st, const EwrArgs<real> &ew, int ignore_intra,
+                                         int use_mol) {
+  using real4 = typename V4<real>::t;
+  const int T = s.n_types;
+  const real4 xi = x4[i];
+  ti = type_of(xi.w);
+  const bool um = !ONE_TYPE && use_mol;  // the single-type instantiation runs without molecules
+  const int moli = um ? s.mol[i] : 0;
+  const int cnt = s.ncount[i];
+  const PairCoef<real> *ci = coef + (ONE_TYPE ? 0 : ti * T);
+  PairCoef<real> c1;
+  if (ONE_TYPE) c1 = coef[0];
+  if (TPA == 1) {
+    // one lane per atom: entries in quads, one 16-byte load per four; the
+    // next quad is loaded before this one's neighbours are gathered, so
+    // the list stream's HBM latency overlaps the gathers and the math.
+    // Full quads need no per-entry count test; the last, partial one does.
+    const uint4 *q4 = reinterpret_cast<const uint4 *>(s.nlist) + i;
+    uint4 nxt = make_uint4(0u, 0u, 0u, 0u);
+    if (cnt > 0) nxt = __ldcs(q4);
+    const int full = cnt & ~3;
+    auto quad = [&](const uint4 &e4, int nv, auto check) {
+      constexpr bool CHECK = decltype(check)::value;
+      const uint32_t e[4] = {e4.x, e4.y, e4.z, e4.w};
+      real4 xj[4];
+      bool sm[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int j = (!CHECK || u < nv) ? (int)(e[u] & INDEX_MASK) : i;
+        xj[u] = x4[j];
+        sm[u] = um && (moli == s.mol[j]);
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        if (!CHECK || u < nv) {
+          real dx, dy, dz;
+          pair_disp<real, FIXED>(xj[u], xi, e[u], st, dx, dy, dz);
+          pair_term<real, LJ, EWR, EV, !ONE_TYPE>(A, dx, dy, dz, ONE_TYPE ? c1 : ci[type_of(xj[u].w)], sm[u], ignore_intra,
+                                       ew);
+        }
+      }
+      if (EV) ev_flush<LJ, EWR>(A);
+    };
+    for (int k = 0; k < full; k += 4) {
+      const uint4 e4 = nxt;
+      q4 += s.n_pad;
+      if (k + 4 < cnt) nxt = __ldcs(q4);
+      quad(e4, 4, std::false_type{});
+    }
+    if (cnt > full) quad(nxt, cnt - full, std::true_type{});
+  } else {
+    const size_t stride = (size_t)s.n_pad * TPA;
+    const uint32_t *row = s.nlist + (size_t)i * TPA + lane;
+    constexpr int U = CVR_PAIR_UNROLL;
+    int k = lane;
+    for (; k + (U - 1) * TPA < cnt; k += U * TPA) {
+      uint32_t e[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) e[u] = __ldcs(row + u * stride);
+      row += U * stride;
+      real4 xj[U];
+      bool sm[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int j = (int)(e[u] & INDEX_MASK);
+        xj[u] = x4[j];
+        sm[u] = um && (moli == s.mol[j]);
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        real dx, dy, dz;
+        pair_disp<real, FIXED>(xj[u], xi, e[u], st, dx, dy, dz);
+        pair_term<real, LJ, EWR, EV, !ONE_TYPE>(A, dx, dy, dz, ONE_TYPE ? c1 : ci[type_of(xj[u].w)], sm[u], ignore_intra,
+                                     ew);
+      }
+      if (EV) ev_flush<LJ, EWR>(A);
+    }
+    for (; k < cnt; k += TPA) {
+      const uint32_t e0 = __ldcs(row);
+      row += stride;
+      const int j0 = (int)(e0 & INDEX_MASK);
+      const real4 xj0 = x4[j0];
+      const bool sm0 = um && (moli == s.mol[j0]);
+      real dx, dy, dz;
+      pair_disp<real, FIXED>(xj0, xi, e0, st, dx, dy, dz);
+      pair_term<real, LJ, EWR, EV, !ONE_TYPE>(A, dx, dy, dz, ONE_TYPE ? c1 : ci[type_of(xj0.w)], sm0, ignore_intra, ew);
+    }
+    if (EV) ev_flush<LJ, EWR>(A);
+  }
+}
+
+template <typename real>
+__device__ __forceinline__ Stencil<real> stencil_of(const DevState<real> &s) {
+  Stencil<real> st;
+  st.bias = (real)(sizeof(real) == 4 ? 8388608.0 : 4503599627370496.0) + (real)s.cells.R;
+  st.wx = (real)s.cells.w[0];
+  st.wy = (real)s.cells.w[1];
+  st.wz = (real)s.cells.w[2];
+  return st;
+}
+
 // FIXED: x4 holds fixed-point coordinates; coef_g and ew are in units of
 // L / 2^32 and fscale = 2^32 / L turns the summed force back into length
 // units (the virial and energies come out unscaled).  Otherwise fscale = 1.
@@ -229,15 +335,10 @@ __global__ void __launch_bounds__(128, CVR_PAIR_MINB) k_pair(DevState<real> s, c
     *s.flag = 0;
     if (counters) counters[0]++;
   }
-  using real4 = typename V4<real>::t;
   __shared__ PairCoef<real> coef[ONE_TYPE ? 1 : MAX_TYPES * MAX_TYPES];
   const int T = s.n_types;
   for (int t = threadIdx.x; t < (ONE_TYPE ? 1 : T * T); t += blockDim.x) coef[t] = coef_g[t];
-  Stencil<real> st;
-  st.bias = (real)(sizeof(real) == 4 ? 8388608.0 : 4503599627370496.0) + (real)s.cells.R;
-  st.wx = (real)s.cells.w[0];
-  st.wy = (real)s.cells.w[1];
-  st.wz = (real)s.cells.w[2];
+  const Stencil<real> st = stencil_of(s);
   __syncthreads();
   if (*s.err) return;
 
@@ -246,93 +347,8 @@ __global__ void __launch_bounds__(128, CVR_PAIR_MINB) k_pair(DevState<real> s, c
   const bool valid = i < s.n;
   PairAcc<real> A{0, 0, 0, 0.0, 0.0, 0.0, 0, 0, 0};
   int ti = 0;
-  if (valid) {
-    const real4 xi = s.x4[i];
-    ti = type_of(xi.w);
-    const bool um = !ONE_TYPE && use_mol;  // the single-type instantiation runs without molecules
-    const int moli = um ? s.mol[i] : 0;
-    const int cnt = s.ncount[i];
-    const PairCoef<real> *ci = coef + (ONE_TYPE ? 0 : ti * T);
-    PairCoef<real> c1;
-    if (ONE_TYPE) c1 = coef[0];
-    if (TPA == 1) {
-      // one lane per atom: entries in quads, one 16-byte load per four; the
-      // next quad is loaded before this one's neighbours are gathered, so
-      // the list stream's HBM latency overlaps the gathers and the math.
-      // Full quads need no per-entry count test; the last, partial one does.
-      const uint4 *q4 = reinterpret_cast<const uint4 *>(s.nlist) + i;
-      uint4 nxt = make_uint4(0u, 0u, 0u, 0u);
-      if (cnt > 0) nxt = __ldcs(q4);
-      const int full = cnt & ~3;
-      auto quad = [&](const uint4 &e4, int nv, auto check) {
-        constexpr bool CHECK = decltype(check)::value;
-        const uint32_t e[4] = {e4.x, e4.y, e4.z, e4.w};
-        real4 xj[4];
-        bool sm[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int j = (!CHECK || u < nv) ? (int)(e[u] & INDEX_MASK) : i;
-          xj[u] = s.x4[j];
-          sm[u] = um && (moli == s.mol[j]);
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          if (!CHECK || u < nv) {
-            real dx, dy, dz;
-            pair_disp<real, FIXED>(xj[u], xi, e[u], st, dx, dy, dz);
-            pair_term<real, LJ, EWR, EV, !ONE_TYPE>(A, dx, dy, dz, ONE_TYPE ? c1 : ci[type_of(xj[u].w)], sm[u], ignore_intra,
-                                         ew);
-          }
-        }
-        if (EV) ev_flush<LJ, EWR>(A);
-      };
-      for (int k = 0; k < full; k += 4) {
-        const uint4 e4 = nxt;
-        q4 += s.n_pad;
-        if (k + 4 < cnt) nxt = __ldcs(q4);
-        quad(e4, 4, std::false_type{});
-      }
-      if (cnt > full) quad(nxt, cnt - full, std::true_type{});
-    } else {
-      const size_t stride = (size_t)s.n_pad * TPA;
-      const uint32_t *row = s.nlist + (size_t)i * TPA + lane;
-      constexpr int U = CVR_PAIR_UNROLL;
-      int k = lane;
-      for (; k + (U - 1) * TPA < cnt; k += U * TPA) {
-        uint32_t e[U];
-#pragma unroll
-        for (int u = 0; u < U; ++u) e[u] = __ldcs(row + u * stride);
-        row += U * stride;
-        real4 xj[U];
-        bool sm[U];
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-          const int j = (int)(e[u] & INDEX_MASK);
-          xj[u] = s.x4[j];
-          sm[u] = um && (moli == s.mol[j]);
-        }
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-          real dx, dy, dz;
-          pair_disp<real, FIXED>(xj[u], xi, e[u], st, dx, dy, dz);
-          pair_term<real, LJ, EWR, EV, !ONE_TYPE>(A, dx, dy, dz, ONE_TYPE ? c1 : ci[type_of(xj[u].w)], sm[u], ignore_intra,
-                                       ew);
-        }
-        if (EV) ev_flush<LJ, EWR>(A);
-      }
-      for (; k < cnt; k += TPA) {
-        const uint32_t e0 = __ldcs(row);
-        row += stride;
-        const int j0 = (int)(e0 & INDEX_MASK);
-        const real4 xj0 = s.x4[j0];
-        const bool sm0 = um && (moli == s.mol[j0]);
-        real dx, dy, dz;
-        pair_disp<real, FIXED>(xj0, xi, e0, st, dx, dy, dz);
-        pair_term<real, LJ, EWR, EV, !ONE_TYPE>(A, dx, dy, dz, ONE_TYPE ? c1 : ci[type_of(xj0.w)], sm0, ignore_intra, ew);
-      }
-      if (EV) ev_flush<LJ, EWR>(A);
-    }
-  }
+  if (valid)
+    pair_row<real, TPA, LJ, EWR, EV, ONE_TYPE, FIXED>(A, ti, s, s.x4, i, lane, coef, st, ew, ignore_intra, use_mol);
 #pragma unroll
   for (int o = TPA / 2; o > 0; o >>= 1) {
     A.fx += __shfl_xor_sync(0xffffffffu, A.fx, o);
@@ -950,7 +966,8 @@ __global__ void __launch_bounds__(512, sizeof(real) == 4 ? CVR_KF_MINB : 1) k_kf
 // After a position update of atom i (cell order) to p: the cell-local
 // coordinates for the pair kernel, and whether the list must be rebuilt.
 template <typename real>
-__device__ __forceinline__ bool update_local(DevState<real> &s, int i, const double (&p)[3]) {
+__device__ __forceinline__ bool update_local(const DevState<real> &s, int i, const double (&p)[3],
+                                             const typename V4<real>::t *x4_in, typename V4<real>::t *x4_out) {
   bool need = false;
   int code = 0, mul = 1;
   if (s.policy == 1) {
@@ -975,12 +992,12 @@ __device__ __forceinline__ bool update_local(DevState<real> &s, int i, const dou
   if (!fx) {
     int cc[3];
     cell_xyz(s, s.cell[i], cc[0], cc[1], cc[2]);
-    q = s.x4[i];
+    q = x4_in[i];
     q.x = (real)(p[0] - (s.box.lo[0] + (cc[0] + 0.5) * s.cells.w[0]));
     q.y = (real)(p[1] - (s.box.lo[1] + (cc[1] + 0.5) * s.cells.w[1]));
     q.z = (real)(p[2] - (s.box.lo[2] + (cc[2] + 0.5) * s.cells.w[2]));
   }
-  s.x4[i] = q;
+  x4_out[i] = q;
   const float4 b = s.xb[i];
   const float ex = (float)(p[0] - s.box.ctr[0]) - b.x, ey = (float)(p[1] - s.box.ctr[1]) - b.y,
               ez = (float)(p[2] - s.box.ctr[2]) - b.z;
@@ -988,6 +1005,42 @@ __device__ __forceinline__ bool update_local(DevState<real> &s, int i, const dou
   if (s.policy == 1 && code != s.gcls[i]) need = true;  // ghost set changed
   if (s.policy == 2) need = true;
   return need;
+}
+
+// Kick and drift of atom i with acceleration a: the velocity u at the
+// step's start (pre_h != 0: after the previous step's second half kick), the
+// half-kicked v and the new position p.
+template <typename real>
+__device__ __forceinline__ void kick_drift_atom(const DevState<real> &s, int i, double dt, double pre_h, double a0,
+                                                double a1, double a2, double (&v)[3], double (&p)[3]) {
+  const double h = 0.5 * dt;
+  double u0 = s.vx[i], u1 = s.vy[i], u2 = s.vz[i];
+  if (pre_h != 0.0) {
+    u0 = u0 + pre_h * a0;
+    u1 = u1 + pre_h * a1;
+    u2 = u2 + pre_h * a2;
+  }
+  v[0] = u0 + h * a0;
+  v[1] = u1 + h * a1;
+  v[2] = u2 + h * a2;
+  p[0] = s.x[i] + dt * v[0];
+  p[1] = s.y[i] + dt * v[1];
+  p[2] = s.z[i] + dt * v[2];
+}
+
+// Stores them and writes the new pair coordinates; true if the list must be rebuilt.
+template <typename real>
+__device__ __forceinline__ bool store_drift(const DevState<real> &s, int i, const double (&a)[3], const double (&v)[3],
+                                            const double (&p)[3], const typename V4<real>::t *x4_in,
+                                            typename V4<real>::t *x4_out) {
+  if (isnan(a[0]) || isnan(a[1]) || isnan(a[2])) atomicOr(s.err, ERR_NAN);  // md_simulator.cpp:584-590
+  s.vx[i] = v[0];
+  s.vy[i] = v[1];
+  s.vz[i] = v[2];
+  s.x[i] = p[0];
+  s.y[i] = p[1];
+  s.z[i] = p[2];
+  return update_local(s, i, p, x4_in, x4_out);
 }
 
 #ifndef KD_PHASE_SUB
@@ -1011,26 +1064,10 @@ __global__ void __launch_bounds__(256) k_kick_drift(DevState<real> s, double dt,
   const int i = t / SUB, sub = t - i * SUB;
   bool need = false;
   if (i < s.n) {
-    const double a0 = (double)s.ax[i], a1 = (double)s.ay[i], a2 = (double)s.az[i];
-    const double h = 0.5 * dt;
-    double u0 = s.vx[i], u1 = s.vy[i], u2 = s.vz[i];
-    if (pre_h != 0.0) {
-      u0 = u0 + pre_h * a0;
-      u1 = u1 + pre_h * a1;
-      u2 = u2 + pre_h * a2;
-    }
-    const double v0 = u0 + h * a0, v1 = u1 + h * a1, v2 = u2 + h * a2;
-    const double p[3] = {s.x[i] + dt * v0, s.y[i] + dt * v1, s.z[i] + dt * v2};
-    if (sub == 0) {
-      if (isnan(a0) || isnan(a1) || isnan(a2)) atomicOr(s.err, ERR_NAN);  // md_simulator.cpp:584-590
-      s.vx[i] = v0;
-      s.vy[i] = v1;
-      s.vz[i] = v2;
-      s.x[i] = p[0];
-      s.y[i] = p[1];
-      s.z[i] = p[2];
-      need = update_local(s, i, p);
-    }
+    const double a[3] = {(double)s.ax[i], (double)s.ay[i], (double)s.az[i]};
+    double v[3], p[3];
+    kick_drift_atom(s, i, dt, pre_h, a[0], a[1], a[2], v, p);
+    if (sub == 0) need = store_drift(s, i, a, v, p, s.x4, s.x4);
     if constexpr (PHASE) {
       if (sub < 3) {
         const double pd = (sub == 0) ? p[0] : ((sub == 1) ? p[1] : p[2]);  // static indices: p stays in registers
@@ -1119,7 +1156,7 @@ __global__ void __launch_bounds__(256) k_lgv_kick_drift(DevState<real> s, double
     s.x[i] = p[0];
     s.y[i] = p[1];
     s.z[i] = p[2];
-    need = update_local(s, i, p);
+    need = update_local(s, i, p, s.x4, s.x4);
   }
   if (__any_sync(0xffffffffu, need) && (threadIdx.x & 31) == 0) *s.flag = 1;
 }
@@ -1211,6 +1248,32 @@ struct ThermostatArgs {
   double *scal;               // [0] Berendsen factor of this step (1 = none), [1] zeta
 };
 
+// The step's Berendsen factor or the Euler step of zeta, from sum m v^2, sum m v.
+__device__ __forceinline__ void thermostat_update(const ThermostatArgs &a, const double (&sums)[4], long long timestep,
+                                                  double &lambda, double &zeta) {
+  double ke = 0.5 * sums[0];
+  if (a.com_removed && a.total_mass > 0)
+    ke -= 0.5 * (sums[1] * sums[1] + sums[2] * sums[2] + sums[3] * sums[3]) / a.total_mass;
+  const double T = (a.dof > 0) ? 2.0 * ke / (a.k_b * a.dof) : 0.0;
+  if (a.kind == 1) {
+    double lam = 1.0;
+    if (timestep % a.every == 0) {
+      lam = sqrt(1.0 + (a.dt / a.tau) * ((a.T0 / T) - 1.0));
+      if (lam < a.lambda_min) lam = a.lambda_min;
+      if (lam > a.lambda_max) lam = a.lambda_max;
+    }
+    lambda = lam;
+  } else {
+    const double g = a.dof;
+    double zd;
+    if (a.nh_type == 1)
+      zd = (-a.nh_kb * a.dof * T / a.nh_mass) * ((g * a.T0 / (a.dof * T)) - 1.0);
+    else
+      zd = (-1.0 / a.nh_tau) * ((g * a.T0 / (a.dof * T)) - 1.0);
+    zeta += a.dt * zd;
+  }
+}
+
 __global__ void __launch_bounds__(256) k_thermostat_coef(ThermostatArgs a) {
   __shared__ double acc[4][256];
   double v[4] = {0, 0, 0, 0};
@@ -1224,28 +1287,8 @@ __global__ void __launch_bounds__(256) k_thermostat_coef(ThermostatArgs a) {
     __syncthreads();
   }
   if (threadIdx.x != 0) return;
-  double ke = 0.5 * acc[0][0];
-  if (a.com_removed && a.total_mass > 0)
-    ke -= 0.5 * (acc[1][0] * acc[1][0] + acc[2][0] * acc[2][0] + acc[3][0] * acc[3][0]) / a.total_mass;
-  const double T = (a.dof > 0) ? 2.0 * ke / (a.k_b * a.dof) : 0.0;
-  const long long timestep = a.counters[0] - 1;  // the reference's current_step of this step
-  if (a.kind == 1) {
-    double lam = 1.0;
-    if (timestep % a.every == 0) {
-      lam = sqrt(1.0 + (a.dt / a.tau) * ((a.T0 / T) - 1.0));
-      if (lam < a.lambda_min) lam = a.lambda_min;
-      if (lam > a.lambda_max) lam = a.lambda_max;
-    }
-    a.scal[0] = lam;
-  } else {
-    const double g = a.dof;
-    double zd;
-    if (a.nh_type == 1)
-      zd = (-a.nh_kb * a.dof * T / a.nh_mass) * ((g * a.T0 / (a.dof * T)) - 1.0);
-    else
-      zd = (-1.0 / a.nh_tau) * ((g * a.T0 / (a.dof * T)) - 1.0);
-    a.scal[1] += a.dt * zd;  // Euler step of zeta
-  }
+  const double sums[4] = {acc[0][0], acc[1][0], acc[2][0], acc[3][0]};
+  thermostat_update(a, sums, a.counters[0] - 1, a.scal[0], a.scal[1]);  // the reference's current_step of this step
 }
 
 // Berendsen: v *= lambda (with KE partials of the scaled velocities for the
@@ -1586,6 +1629,33 @@ struct ThermoArgs {
   double *out;          // base of the records, CVR_N_THERMO doubles each
 };
 
+// One record from the sums acc = {sum m v^2, sum m v (3), e_lj, e_ewr, virial, sum f_k |S_k|^2}.
+__device__ __forceinline__ void thermo_record(const ThermoArgs &a, const double (&acc)[8], long long step, double *out) {
+  const double mv2 = acc[0];
+  double ke = 0.5 * mv2;
+  if (a.com_removed && a.total_mass > 0) {
+    const double px = acc[1], py = acc[2], pz = acc[3];
+    ke -= 0.5 * (px * px + py * py + pz * pz) / a.total_mass;
+  }
+  const double temp = (a.dof > 0) ? 2.0 * ke / (a.k_b * a.dof) : 0.0;
+  const double vir = acc[6];
+  out[0] = (double)step;
+  out[1] = ke;
+  out[2] = temp;
+  out[3] = acc[4];
+  out[4] = acc[5];
+  out[5] = a.ek_coef * acc[7];
+  if (a.dipole) {
+    const double *M = a.dipole + 3;
+    out[5] += 0.5 * a.dipole_coef * (M[0] * M[0] + M[1] * M[1] + M[2] * M[2]);
+  }
+  if (a.slab_e) out[5] += *a.slab_e;
+  out[6] = a.e_self;
+  out[7] = vir;
+  out[8] = a.n_atoms * a.k_b * temp / a.volume + vir / (3.0 * a.volume);
+  out[9] = (double)(*a.n_builds);
+}
+
 // One block of THERMO_THREADS: each thread sums its strided share of the
 // block partials (loops unrolled so that several loads are in flight), then
 // warp shuffles and one warp finish the sums (a fixed order).
@@ -1625,31 +1695,8 @@ __global__ void __launch_bounds__(THERMO_THREADS) k_thermo(ThermoArgs a) {
     acc[q] = x;
   }
   if (lane == 0) {
-    const long long rec = a.counters[1]++;
-    double *out = a.out + rec * 10;
-    const double mv2 = acc[0];
-    double ke = 0.5 * mv2;
-    if (a.com_removed && a.total_mass > 0) {
-      const double px = acc[1], py = acc[2], pz = acc[3];
-      ke -= 0.5 * (px * px + py * py + pz * pz) / a.total_mass;
-    }
-    const double temp = (a.dof > 0) ? 2.0 * ke / (a.k_b * a.dof) : 0.0;
-    const double vir = acc[6];
-    out[0] = (double)a.counters[0];
-    out[1] = ke;
-    out[2] = temp;
-    out[3] = acc[4];
-    out[4] = acc[5];
-    out[5] = a.ek_coef * acc[7];
-    if (a.dipole) {
-      const double *M = a.dipole + 3;
-      out[5] += 0.5 * a.dipole_coef * (M[0] * M[0] + M[1] * M[1] + M[2] * M[2]);
-    }
-    if (a.slab_e) out[5] += *a.slab_e;
-    out[6] = a.e_self;
-    out[7] = vir;
-    out[8] = a.n_atoms * a.k_b * temp / a.volume + vir / (3.0 * a.volume);
-    out[9] = (double)(*a.n_builds);
+    thermo_record(a, acc, a.counters[0], a.out + a.counters[1] * 10);
+    a.counters[1]++;
   }
 }
 
