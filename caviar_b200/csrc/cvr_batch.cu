@@ -596,6 +596,94 @@ __global__ void __launch_bounds__(TPB, 1) k_batch(BatchDev p, int first, int nst
   }
 }
 
+// ---------------------------------------------------- state in and out
+// The caller's arrays are AoS in atom order; the stored ones SoA with each
+// replica's charged atoms first.  Both reorderings run here, on the staged
+// upload and before the download: on the host they took 60 ms for a million
+// atoms (1024 replicas) beside 25 ms of transfers (pageable memory).
+
+// Types out of range (counted into *bad).
+__global__ void __launch_bounds__(256) k_batch_check(const int *__restrict__ type, long long n, int n_types,
+                                                     unsigned *__restrict__ bad) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const bool out = i < n && (type[i] < 0 || type[i] >= n_types);
+  if (__syncthreads_or(out) && threadIdx.x == 0) atomicAdd(bad, 1u);
+}
+
+// One block per replica: the stored slot of each atom (charged atoms first,
+// each kind in the caller's order) by a block-wide count, then the scatter.
+constexpr int PLACE_THREADS = 256;
+__global__ void __launch_bounds__(PLACE_THREADS) k_batch_place(BatchDev p, const double *__restrict__ pos,
+                                                               const double *__restrict__ vel,
+                                                               const int *__restrict__ type, int *__restrict__ slot_of,
+                                                               int *__restrict__ type_out, int *__restrict__ nq_out) {
+  __shared__ int warp_q[PLACE_THREADS / 32];
+  const int r = blockIdx.x, n = p.n[r], lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const long long o = p.off[r];
+  // charged atoms of the replica
+  int mine = 0;
+  for (int i = threadIdx.x; i < n; i += PLACE_THREADS) mine += p.chargeD[type[o + i]] != 0.0;
+  mine = __reduce_add_sync(0xffffffffu, mine);
+  if (lane == 0) warp_q[warp] = mine;
+  __syncthreads();
+  int nq = 0;
+  for (int w = 0; w < PLACE_THREADS / 32; ++w) nq += warp_q[w];
+  if (threadIdx.x == 0) nq_out[r] = nq;
+  int before = 0;  // charged atoms before this round
+  for (int base = 0; base < n; base += PLACE_THREADS) {
+    const int i = base + threadIdx.x;
+    const int t = i < n ? type[o + i] : 0;
+    const bool q = i < n && p.chargeD[t] != 0.0;
+    const unsigned m = __ballot_sync(0xffffffffu, q);
+    __syncthreads();
+    if (lane == 0) warp_q[warp] = __popc(m);
+    __syncthreads();
+    int ahead = before, all = 0;
+    for (int w = 0; w < PLACE_THREADS / 32; ++w) {
+      if (w < warp) ahead += warp_q[w];
+      all += warp_q[w];
+    }
+    ahead += __popc(m & ((1u << lane) - 1u));  // charged atoms before atom i
+    before += all;
+    if (i < n) {
+      const long long s = o + (q ? ahead : nq + i - ahead), a = o + i;
+      slot_of[a] = (int)s;
+      type_out[s] = t;
+      p.x[s] = pos[3 * a];
+      p.y[s] = pos[3 * a + 1];
+      p.z[s] = pos[3 * a + 2];
+      p.vx[s] = vel ? vel[3 * a] : 0.0;
+      p.vy[s] = vel ? vel[3 * a + 1] : 0.0;
+      p.vz[s] = vel ? vel[3 * a + 2] : 0.0;
+    }
+  }
+}
+
+// Stored values back to the caller's order (each output nullable); acc = F/m.
+__global__ void __launch_bounds__(256) k_batch_gather(BatchDev p, long long n, const int *__restrict__ slot_of,
+                                                      double *__restrict__ pos, double *__restrict__ vel,
+                                                      double *__restrict__ acc) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const long long s = slot_of ? slot_of[i] : i;
+  if (pos) {
+    pos[3 * i] = p.x[s];
+    pos[3 * i + 1] = p.y[s];
+    pos[3 * i + 2] = p.z[s];
+  }
+  if (vel) {
+    vel[3 * i] = p.vx[s];
+    vel[3 * i + 1] = p.vy[s];
+    vel[3 * i + 2] = p.vz[s];
+  }
+  if (acc) {
+    const double mi = p.mass_inv[p.type[s]];
+    acc[3 * i] = (double)p.fx[s] * mi;
+    acc[3 * i + 1] = (double)p.fy[s] * mi;
+    acc[3 * i + 2] = (double)p.fz[s] * mi;
+  }
+}
+
 using KernelFn = void (*)(BatchDev, int, int, int, int, int);
 
 struct Shape {
@@ -617,11 +705,13 @@ struct cvr_batch {
   cudaStream_t stream = nullptr;
   int n_rep = 0, n_types = 0;
   long long n_total = 0;
-  std::vector<int> n, nq;
+  std::vector<int> n;
   std::vector<long long> off;
   std::vector<double> L, rc_lj, rc_r;
-  std::vector<int> slot_of;  // caller's atom index -> stored slot (charged atoms first within a replica)
-  std::vector<double> charge_h;
+  int *slot_of = nullptr;    // device: caller's atom index -> stored slot (charged atoms first within a replica)
+  double *stage = nullptr;   // device: 9 doubles per atom, the caller's layout
+  int *stage_type = nullptr; // device, and one counter behind it
+  bool have_state = false;
   bool uniform = false;      // every type pair has the same eps and sigma
   BatchDev dev{};
   std::vector<void *> allocs;
@@ -632,8 +722,9 @@ struct cvr_batch {
   std::vector<Class> classes;
   cudaStream_t side[3] = {nullptr, nullptr, nullptr};  // one per size class: the graph's parallel branches
   cudaEvent_t fork = nullptr, join[3] = {nullptr, nullptr, nullptr};
-  cudaGraphExec_t graph = nullptr;
-  int graph_steps = -1;
+  // one graph per (nsteps, forces of the first positions computed in the launch)
+  cudaGraphExec_t graph[2] = {nullptr, nullptr};
+  int graph_steps[2] = {-1, -1};
   std::string err;
   bool tuned = false;
   bool forces_valid = false;  // fx/fy/fz hold the forces of the current positions
@@ -683,9 +774,7 @@ int cvr_batch_create(cvr_batch **out, int n_rep, const int64_t *n_atoms, const d
   b->n_rep = n_rep;
   b->n_types = n_types;
   b->n.assign(n_atoms, n_atoms + n_rep);
-  b->nq.assign(n_rep, 0);
   b->L.assign(box_len, box_len + n_rep);
-  b->charge_h.assign(charge, charge + n_types);
   b->off.resize(n_rep);
   long long o = 0;
   for (int r = 0; r < n_rep; ++r) {
@@ -721,7 +810,8 @@ int cvr_batch_create(cvr_batch **out, int n_rep, const int64_t *n_atoms, const d
   int *dtype;
   double *dout;
   if ((rc = balloc(b, &arr, 6 * N)) || (rc = balloc(b, &farr, 3 * N)) || (rc = balloc(b, &dtype, N)) ||
-      (rc = balloc(b, &dout, (size_t)n_rep * NTH)))
+      (rc = balloc(b, &dout, (size_t)n_rep * NTH)) || (rc = balloc(b, &b->slot_of, N)) ||
+      (rc = balloc(b, &b->stage, 9 * N)) || (rc = balloc(b, &b->stage_type, N + 1)))
     return rc;
   d.x = arr;
   d.y = arr + N;
@@ -730,6 +820,7 @@ int cvr_batch_create(cvr_batch **out, int n_rep, const int64_t *n_atoms, const d
   d.vy = arr + 4 * N;
   d.vz = arr + 5 * N;
   cudaMemset(farr, 0, 3 * N * sizeof(float));
+  cudaMemset(dtype, 0, N * sizeof(int));
   d.fx = farr;
   d.fy = farr + N;
   d.fz = farr + 2 * N;
@@ -767,7 +858,8 @@ void cvr_batch_destroy(cvr_batch *b) {
   if (!b) return;
   cudaSetDevice(b->device);
   cudaStreamSynchronize(b->stream);
-  if (b->graph) cudaGraphExecDestroy(b->graph);
+  for (cudaGraphExec_t g : b->graph)
+    if (g) cudaGraphExecDestroy(g);
   for (void *p : b->allocs) cudaFree(p);
   for (int c = 0; c < 3; ++c) {
     cudaStreamDestroy(b->side[c]);
@@ -863,10 +955,11 @@ int cvr_batch_set_forces(cvr_batch *b, const double *eps, const double *sigma, c
   }
   b->tuned = false;
   b->forces_valid = false;
-  if (b->graph) {
-    cudaGraphExecDestroy(b->graph);
-    b->graph = nullptr;
-  }
+  for (cudaGraphExec_t &g : b->graph)
+    if (g) {
+      cudaGraphExecDestroy(g);
+      g = nullptr;
+    }
   return CVR_OK;
 }
 
@@ -874,38 +967,24 @@ int cvr_batch_set_state(cvr_batch *b, const double *pos, const double *vel, cons
   if (!b || !pos || !type) return CVR_ERR_INVALID;
   cudaSetDevice(b->device);
   const size_t N = (size_t)b->n_total;
-  for (size_t i = 0; i < N; ++i)
-    if (type[i] < 0 || type[i] >= b->n_types) return bfail(b, CVR_ERR_INVALID, "atom type out of range");
-  // within each replica, charged atoms first (stable): the pair tiles then
-  // know from the block index alone whether Ewald terms can occur
-  b->slot_of.assign(N, 0);
-  for (int r = 0; r < b->n_rep; ++r) {
-    const long long o = b->off[r];
-    int k = 0;
-    for (int pass = 0; pass < 2; ++pass)
-      for (int i = 0; i < b->n[r]; ++i) {
-        const bool charged = b->charge_h[type[o + i]] != 0.0;
-        if (charged == (pass == 0)) b->slot_of[o + i] = (int)(o + k++);
-      }
-    int q = 0;
-    for (int i = 0; i < b->n[r]; ++i) q += b->charge_h[type[o + i]] != 0.0;
-    b->nq[r] = q;
-  }
-  std::vector<double> soa(6 * N, 0.0);
-  std::vector<int32_t> ts(N);
-  for (size_t i = 0; i < N; ++i) {
-    const size_t sl = (size_t)b->slot_of[i];
-    ts[sl] = type[i];
-    for (int a = 0; a < 3; ++a) {
-      soa[a * N + sl] = pos[3 * i + a];
-      soa[(3 + a) * N + sl] = vel ? vel[3 * i + a] : 0.0;
-    }
-  }
-  cudaMemcpyAsync(b->dev.x, soa.data(), 6 * N * sizeof(double), cudaMemcpyHostToDevice, b->stream);
-  cudaMemcpyAsync((void *)b->dev.type, ts.data(), N * sizeof(int32_t), cudaMemcpyHostToDevice, b->stream);
-  cudaMemcpyAsync((void *)b->dev.nq, b->nq.data(), b->n_rep * sizeof(int), cudaMemcpyHostToDevice, b->stream);
+  unsigned *bad = reinterpret_cast<unsigned *>(b->stage_type + N), n_bad = 0;
+  cudaStream_t st = b->stream;
+  // the stored state changes only after the types are known to be in range
+  cudaMemcpyAsync(b->stage_type, type, N * sizeof(int32_t), cudaMemcpyHostToDevice, st);
+  cudaMemsetAsync(bad, 0, sizeof(unsigned), st);
+  k_batch_check<<<(unsigned)((N + 255) / 256), 256, 0, st>>>(b->stage_type, (long long)N, b->n_types, bad);
+  cudaMemcpyAsync(&n_bad, bad, sizeof(unsigned), cudaMemcpyDeviceToHost, st);
+  cudaMemcpyAsync(b->stage, pos, 3 * N * sizeof(double), cudaMemcpyHostToDevice, st);
+  if (vel) cudaMemcpyAsync(b->stage + 3 * N, vel, 3 * N * sizeof(double), cudaMemcpyHostToDevice, st);
+  if (cudaStreamSynchronize(st) != cudaSuccess) return bfail(b, CVR_ERR_CUDA, "upload");
+  if (n_bad) return bfail(b, CVR_ERR_INVALID, "atom type out of range");
+  k_batch_place<<<b->n_rep, PLACE_THREADS, 0, st>>>(b->dev, b->stage, vel ? b->stage + 3 * N : nullptr, b->stage_type,
+                                                    b->slot_of, const_cast<int *>(b->dev.type),
+                                                    const_cast<int *>(b->dev.nq));
   b->forces_valid = false;
-  return cudaStreamSynchronize(b->stream) == cudaSuccess ? CVR_OK : bfail(b, CVR_ERR_CUDA, "upload");
+  b->have_state = true;
+  const cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? CVR_OK : bfail(b, CVR_ERR_CUDA, cudaGetErrorString(e));
 }
 
 // Autotuner: for each size class, time every launch shape (threads per CTA,
@@ -963,18 +1042,16 @@ int cvr_batch_run(cvr_batch *b, int64_t nsteps, double *out) {
   if (!b) return CVR_ERR_INVALID;
   if (nsteps < 0 || nsteps > (1 << 30)) return bfail(b, CVR_ERR_INVALID, "bad step count");
   if (!b->dev.kint) return bfail(b, CVR_ERR_STATE, "cvr_batch_set_forces has not been called");
-  if (b->slot_of.empty()) return bfail(b, CVR_ERR_STATE, "cvr_batch_set_state has not been called");
+  if (!b->have_state) return bfail(b, CVR_ERR_STATE, "cvr_batch_set_state has not been called");
   cudaSetDevice(b->device);
   if (!b->tuned)
     if (int rc = batch_tune(b)) return rc;
-  if (!b->forces_valid) {
-    for (auto &c : b->classes)
-      if (launch_class(b, c, c.shape, 0, 1, b->stream)) return bfail(b, CVR_ERR_CUDA, "force launch failed");
-    b->forces_valid = true;
-  }
-  if (!b->graph || b->graph_steps != (int)nsteps) {
-    if (b->graph) cudaGraphExecDestroy(b->graph);
-    b->graph = nullptr;
+  // forces of a new state's positions: in the same launch, ahead of the steps
+  const int first = b->forces_valid ? 0 : 1;
+  cudaGraphExec_t &graph = b->graph[first];
+  if (!graph || b->graph_steps[first] != (int)nsteps) {
+    if (graph) cudaGraphExecDestroy(graph);
+    graph = nullptr;
     cudaGraph_t g;
     if (cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess)
       return bfail(b, CVR_ERR_CUDA, "capture");
@@ -984,17 +1061,18 @@ int cvr_batch_run(cvr_batch *b, int64_t nsteps, double *out) {
     cudaEventRecord(b->fork, b->stream);
     for (size_t ci = 0; ci < b->classes.size(); ++ci) {
       cudaStreamWaitEvent(b->side[ci], b->fork, 0);
-      lrc |= launch_class(b, b->classes[ci], b->classes[ci].shape, (int)nsteps, 0, b->side[ci]);
+      lrc |= launch_class(b, b->classes[ci], b->classes[ci].shape, (int)nsteps, first, b->side[ci]);
       cudaEventRecord(b->join[ci], b->side[ci]);
       cudaStreamWaitEvent(b->stream, b->join[ci], 0);
     }
     const cudaError_t ce = cudaStreamEndCapture(b->stream, &g);
     if (ce != cudaSuccess || lrc != CVR_OK) return bfail(b, CVR_ERR_CUDA, "capture of the replica launches failed");
-    if (cudaGraphInstantiate(&b->graph, g, 0) != cudaSuccess) return bfail(b, CVR_ERR_CUDA, "instantiate");
+    if (cudaGraphInstantiate(&graph, g, 0) != cudaSuccess) return bfail(b, CVR_ERR_CUDA, "instantiate");
     cudaGraphDestroy(g);
-    b->graph_steps = (int)nsteps;
+    b->graph_steps[first] = (int)nsteps;
   }
-  if (cudaGraphLaunch(b->graph, b->stream) != cudaSuccess) return bfail(b, CVR_ERR_CUDA, "graph launch");
+  if (cudaGraphLaunch(graph, b->stream) != cudaSuccess) return bfail(b, CVR_ERR_CUDA, "graph launch");
+  b->forces_valid = true;
   if (out)
     cudaMemcpyAsync(out, b->dev.out, (size_t)b->n_rep * NTH * sizeof(double), cudaMemcpyDeviceToHost, b->stream);
   const cudaError_t e = cudaStreamSynchronize(b->stream);
@@ -1006,21 +1084,15 @@ int cvr_batch_get_state(cvr_batch *b, double *pos, double *vel, double *acc) {
   if (!b) return CVR_ERR_INVALID;
   cudaSetDevice(b->device);
   const size_t N = (size_t)b->n_total;
-  std::vector<double> soa(6 * N);
-  std::vector<float> a(3 * N);
-  std::vector<int32_t> t(N);
-  cudaMemcpyAsync(soa.data(), b->dev.x, 6 * N * sizeof(double), cudaMemcpyDeviceToHost, b->stream);
-  cudaMemcpyAsync(a.data(), b->dev.fx, 3 * N * sizeof(float), cudaMemcpyDeviceToHost, b->stream);
-  cudaMemcpyAsync(t.data(), b->dev.type, N * sizeof(int32_t), cudaMemcpyDeviceToHost, b->stream);
+  double *dp = b->stage, *dv = dp + 3 * N, *da = dv + 3 * N;
+  k_batch_gather<<<(unsigned)((N + 255) / 256), 256, 0, b->stream>>>(
+      b->dev, (long long)N, b->have_state ? b->slot_of : nullptr, pos ? dp : nullptr, vel ? dv : nullptr,
+      acc ? da : nullptr);
+  const size_t bytes = 3 * N * sizeof(double);
+  if (pos) cudaMemcpyAsync(pos, dp, bytes, cudaMemcpyDeviceToHost, b->stream);
+  if (vel) cudaMemcpyAsync(vel, dv, bytes, cudaMemcpyDeviceToHost, b->stream);
+  if (acc) cudaMemcpyAsync(acc, da, bytes, cudaMemcpyDeviceToHost, b->stream);
   if (cudaStreamSynchronize(b->stream) != cudaSuccess) return bfail(b, CVR_ERR_CUDA, "download");
-  for (size_t i = 0; i < N; ++i) {
-    const size_t sl = b->slot_of.empty() ? i : (size_t)b->slot_of[i];
-    for (int d = 0; d < 3; ++d) {
-      if (pos) pos[3 * i + d] = soa[d * N + sl];
-      if (vel) vel[3 * i + d] = soa[(3 + d) * N + sl];
-      if (acc) acc[3 * i + d] = (double)a[d * N + sl] * b->dev.mass_inv[t[sl]];
-    }
-  }
   return CVR_OK;
 }
 
