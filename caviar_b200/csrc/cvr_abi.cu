@@ -215,6 +215,14 @@ struct cvr_ctx {
   ThermostatArgs tstat{};
   double *d_tscal{};  // [0] Berendsen factor, [1] Nose-Hoover zeta (carried across calls)
   std::vector<void *> all_allocs;
+  // pinned: what a call reads back with its one synchronisation
+  struct Back {
+    int flags[4];
+    unsigned long long per_type[MAX_TYPES + 1];
+    double thermo[CVR_N_THERMO];
+  } *back = nullptr;
+  int builds_seen = 0;      // list builds (flags[3]) at the last read
+  bool list_fresh = false;  // cvr_set_state built the list: the next run computes its first forces and no list
 };
 
 // ------------------------------------------------------------------ helpers
@@ -982,6 +990,45 @@ void launch_thermo(cvr_ctx *c, double *out) {
   c->launches++;
 }
 
+// A grid for kernels that meet at grid barriers, one block per SM at most
+// (its co-residence is what the barriers need), for `groups` warps of work:
+// every SM down to four warps per block, one per scheduler (a small system's
+// stages are latency chains, which share nothing on an SM of their own).
+struct GridShape {
+  int grid, threads;
+};
+GridShape grid_shape(const cvr_ctx *c, int groups) {
+  GridShape g;
+  g.grid = std::min(c->sms, grid_for(groups, 4));
+  g.threads = std::min(STEP_THREADS, 32 * grid_for(groups, g.grid));
+  return g;
+}
+
+// A list build outside the step loop: one launch (k_build_once) for the
+// systems whose lists a warp per atom searches, else launch_build's.
+template <typename real>
+int launch_build_now(cvr_ctx *c, int count_only) {
+  if (c->timing || c->n > STEPS_MAX_ATOMS || list_kernel_kind(c) != CVR_LIST_WARP) {
+    launch_build<real>(c, count_only);
+    return CVR_OK;
+  }
+  DevState<real> s = dev_state<real>(c);
+  const GridShape g = grid_shape(c, (int)c->n);
+  const size_t smem = steps_smem(g.threads / 32);
+  auto kernel = k_build_once<real>;
+  CVR_CUDA(c, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  int log2_tpa = c->log2_tpa, launch = c->step_launch;
+  c->step_launch ^= 1;
+  void *args[] = {&s, &c->step_ctrl, &launch, &count_only, &log2_tpa};
+  CVR_CUDA(c, cudaLaunchCooperativeKernel((const void *)kernel, dim3(g.grid), dim3(g.threads), args, smem, c->stream));
+  c->launches++;
+  if (phase_in_drift(c)) {  // the atoms moved in memory: the step's phase tables follow them
+    k_phase<real><<<grid_for(3 * (int64_t)c->n, 256), 256, 0, c->stream>>>(s, kargs<real>(c), s.flag);
+    c->launches++;
+  }
+  return CVR_OK;
+}
+
 template <typename real>
 int do_build(cvr_ctx *c, bool force) {
   DevState<real> s = dev_state<real>(c);
@@ -992,7 +1039,7 @@ int do_build(cvr_ctx *c, bool force) {
   if (c->cap == 0) {
     // size the list: count pass, then allocate
     CVR_CUDA(c, cudaMemsetAsync(c->flags + 2, 0, sizeof(int), c->stream));
-    launch_build<real>(c, 1);
+    if (int r = launch_build_now<real>(c, 1)) return r;
     int mc = 0;
     CVR_CUDA(c, cudaMemcpyAsync(&mc, c->flags + 2, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
     CVR_CUDA(c, cudaStreamSynchronize(c->stream));
@@ -1001,13 +1048,18 @@ int do_build(cvr_ctx *c, bool force) {
     CVR_CUDA(c, cudaMemcpyAsync(c->flags, &one, sizeof(int), cudaMemcpyHostToDevice, c->stream));
   }
   CVR_CUDA(c, cudaMemsetAsync(c->flags + 2, 0, sizeof(int), c->stream));
-  launch_build<real>(c, 0);
-  return CVR_OK;
+  return launch_build_now<real>(c, 0);
 }
 
 int read_flags(cvr_ctx *c, int out[4]) {
-  CVR_CUDA(c, cudaMemcpyAsync(out, c->flags, 4 * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+  CVR_CUDA(c, cudaMemcpyAsync(c->back->flags, c->flags, 4 * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
   CVR_CUDA(c, cudaStreamSynchronize(c->stream));
+  if (out != c->back->flags) std::memcpy(out, c->back->flags, 4 * sizeof(int));
+  c->builds_seen = c->back->flags[3];
+  if (c->back->flags[1] & ERR_BARRIER) {  // the barrier words start again from zero
+    cudaMemsetAsync(c->step_ctrl, 0, SC_WORDS * sizeof(unsigned long long), c->stream);
+    return fail(c, CVR_ERR_CUDA, "a grid barrier's wait ran out");
+  }
   return CVR_OK;
 }
 
@@ -1161,11 +1213,19 @@ int snapshot(cvr_ctx *c, bool restore) {
       c->all_allocs.push_back(q);
       p.second = q;
     }
-    if (restore)
-      CVR_CUDA(c, cudaMemcpyAsync(p.first, p.second, c->snap_bytes[k], cudaMemcpyDeviceToDevice, c->stream));
-    else
-      CVR_CUDA(c, cudaMemcpyAsync(p.second, p.first, c->snap_bytes[k], cudaMemcpyDeviceToDevice, c->stream));
   }
+  CopyArgs a{};
+  size_t most = 0;
+  const int n = (int)c->snap_pairs.size();  // 16 arrays (COPY_MAX holds them)
+  for (int k = 0; k < n; ++k) {
+    a.src[k] = restore ? c->snap_pairs[k].second : c->snap_pairs[k].first;
+    a.dst[k] = restore ? c->snap_pairs[k].first : c->snap_pairs[k].second;
+    a.bytes[k] = c->snap_bytes[k];
+    most = std::max(most, a.bytes[k]);
+  }
+  const int blocks = std::max(1, std::min(2 * c->sms, grid_for((int64_t)(most / 16), 256)));
+  k_copy_arrays<<<dim3(blocks, n), 256, 0, c->stream>>>(a);
+  c->launches++;
   return CVR_OK;
 }
 
@@ -1282,12 +1342,7 @@ bool steps_in_one(const cvr_ctx *c) {
 
 template <typename real, int TPA, bool ONE_TYPE, bool FIXED>
 int launch_steps_t(cvr_ctx *c, int nsteps, int64_t every, int64_t done) {
-  // every SM (one block each at most: its co-residence is what the barriers
-  // need) down to four warps per block, one per scheduler: a small system's
-  // stages are latency chains, which share nothing on an SM of their own
-  const int groups = grid_for(c->n, 32 / TPA);
-  const int grid = std::min(c->sms, grid_for(groups, 4));
-  const int threads = std::min(STEP_THREADS, 32 * grid_for(groups, grid));
+  const GridShape g = grid_shape(c, grid_for(c->n, 32 / TPA));
   const double h = FIXED ? c->L[0] / std::ldexp(1.0, 32) : 1.0;  // as launch_pair_t
   StepArgs<real> a{};
   a.coef = (const PairCoef<real> *)c->d_coef;
@@ -1315,11 +1370,11 @@ int launch_steps_t(cvr_ctx *c, int nsteps, int64_t every, int64_t done) {
   a.done = every > 0 ? (int)(done % every) : 0;
   if (every > 0) a.th = thermo_args(c, c->d_thermo);
   DevState<real> s = dev_state<real>(c);
-  const size_t smem = steps_smem(threads / 32);
+  const size_t smem = steps_smem(g.threads / 32);
   auto kernel = k_steps<real, TPA, ONE_TYPE, FIXED>;
   CVR_CUDA(c, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   void *args[] = {&s, &a};
-  CVR_CUDA(c, cudaLaunchCooperativeKernel((const void *)kernel, dim3(grid), dim3(threads), args, smem, c->stream));
+  CVR_CUDA(c, cudaLaunchCooperativeKernel((const void *)kernel, dim3(g.grid), dim3(g.threads), args, smem, c->stream));
   c->launches++;
   return CVR_OK;
 }
@@ -1407,16 +1462,20 @@ int build_graphs(cvr_ctx *c) {
 
 template <typename real>
 int run_impl(cvr_ctx *c, int64_t nsteps, int64_t every, double *thermo) {
-  if (!c->setup_done)
+  if (!c->setup_done && c->list_fresh) {
+    if (int r = forces_now<real>(c, false)) return r;  // its errors are read with the run's
+    c->setup_done = true;
+  } else if (!c->setup_done) {
     if (int r = setup_run<real>(c)) return r;
+  }
+  c->list_fresh = false;
   const int64_t nrec = (every > 0) ? nsteps / every : 0;
   if ((size_t)nrec > c->thermo_cap) {
     if (int r = dalloc(c, &c->d_thermo, (size_t)std::max<int64_t>(nrec, 1) * CVR_N_THERMO)) return r;
     c->thermo_cap = (size_t)nrec;
   }
   if (int r = snapshot(c, false)) return r;
-  int f0[4];
-  if (int r = read_flags(c, f0)) return r;
+  const int builds0 = c->builds_seen;
   const int64_t step0 = c->step;
   std::mt19937 gen0[3];
   std::normal_distribution<double> nd0[3];
@@ -1482,6 +1541,9 @@ int run_impl(cvr_ctx *c, int64_t nsteps, int64_t every, double *thermo) {
       pending = tail == 0;
     }
     int f[4];
+    if (nrec > 0)
+      CVR_CUDA(c, cudaMemcpyAsync(c->back->thermo, c->d_thermo + (nrec - 1) * CVR_N_THERMO,
+                                  CVR_N_THERMO * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     if (int r = read_flags(c, f)) return r;
     collect_timing(c);
     if (graphs && !in_one) {
@@ -1494,11 +1556,7 @@ int run_impl(cvr_ctx *c, int64_t nsteps, int64_t every, double *thermo) {
                        (c->sc_on ? 4 : 0) + ((c->ewk_on && c->dipole_mode) ? 3 : 0);
       const int kick_plain = kick_in_kforce(c, false) ? 0 : 1;
       c->launches = launches0 + nsteps * (2 + tail) + n_kick * kick_plain + nrec * 2 +
-                    (8 + (phase_in_drift(c) ? 1 : 0)) * (int64_t)(f[3] - f0[3]);
-    }
-    if (f[1] & ERR_BARRIER) {
-      cudaMemsetAsync(c->step_ctrl, 0, SC_WORDS * sizeof(unsigned long long), c->stream);
-      return fail(c, CVR_ERR_CUDA, "a grid barrier's wait ran out");
+                    (8 + (phase_in_drift(c) ? 1 : 0)) * (int64_t)(f[3] - builds0);
     }
     if (f[1] & ERR_NAN) return fail(c, CVR_ERR_NAN, "NaN acceleration");
     if (f[1] & ERR_KSPACE_TC) return fail(c, CVR_ERR_CUDA, "tensor-core k-space force: a wait ran out");
@@ -1506,7 +1564,7 @@ int run_impl(cvr_ctx *c, int64_t nsteps, int64_t every, double *thermo) {
       // replay the call from the snapshot with a larger list
       if (int r = snapshot(c, true)) return r;
       if (int r = regrow(c)) return r;
-      CVR_CUDA(c, cudaMemcpyAsync(c->flags + 3, &f0[3], sizeof(int), cudaMemcpyHostToDevice, c->stream));
+      CVR_CUDA(c, cudaMemcpyAsync(c->flags + 3, &builds0, sizeof(int), cudaMemcpyHostToDevice, c->stream));
       if (int r = do_build<real>(c, true)) return r;
       CVR_CUDA(c, cudaMemsetAsync(c->flags, 0, sizeof(int), c->stream));
       if (int r = forces_now<real>(c, false)) return r;
@@ -1514,12 +1572,12 @@ int run_impl(cvr_ctx *c, int64_t nsteps, int64_t every, double *thermo) {
     }
     c->step = step0 + nsteps;
     if (nrec > 0) {
-      if (thermo)
+      std::memcpy(c->last_thermo, c->back->thermo, sizeof(c->last_thermo));
+      if (thermo) {
         CVR_CUDA(c, cudaMemcpyAsync(thermo, c->d_thermo, (size_t)nrec * CVR_N_THERMO * sizeof(double),
                                     cudaMemcpyDeviceToHost, c->stream));
-      CVR_CUDA(c, cudaMemcpyAsync(c->last_thermo, c->d_thermo + (nrec - 1) * CVR_N_THERMO,
-                                  CVR_N_THERMO * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-      CVR_CUDA(c, cudaStreamSynchronize(c->stream));
+        CVR_CUDA(c, cudaStreamSynchronize(c->stream));
+      }
     }
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return fail(c, CVR_ERR_CUDA, std::string("kernel launch: ") + cudaGetErrorString(e));
@@ -1547,7 +1605,7 @@ int compute_impl(cvr_ctx *c, double *acc, double *thermo) {
   c->counter_src[1] = 0;
   CVR_CUDA(c, cudaMemcpyAsync(c->counters, c->counter_src, sizeof(c->counter_src), cudaMemcpyHostToDevice, c->stream));
   launch_thermo(c, c->d_thermo);
-  CVR_CUDA(c, cudaMemcpyAsync(c->last_thermo, c->d_thermo, CVR_N_THERMO * sizeof(double), cudaMemcpyDeviceToHost,
+  CVR_CUDA(c, cudaMemcpyAsync(c->back->thermo, c->d_thermo, CVR_N_THERMO * sizeof(double), cudaMemcpyDeviceToHost,
                               c->stream));
   if (acc) {
     k_gather_state<real><<<grid_for(c->n, 256), 256, 0, c->stream>>>(s, nullptr, nullptr, c->stage);
@@ -1556,6 +1614,7 @@ int compute_impl(cvr_ctx *c, double *acc, double *thermo) {
   }
   int f[4];
   if (int r = read_flags(c, f)) return r;
+  std::memcpy(c->last_thermo, c->back->thermo, sizeof(c->last_thermo));
   collect_timing(c);
   if (f[1] & ERR_OVERFLOW) {
     if (int r = regrow(c)) return r;
@@ -1628,6 +1687,7 @@ int refresh(cvr_ctx *c) {
       set_smem_attrs<float>(c);
   }
   c->list_valid = false;
+  c->list_fresh = false;
   c->setup_done = false;
   c->refreshed = true;
   return CVR_OK;
@@ -1765,11 +1825,12 @@ int cvr_create(cvr_ctx **out, const double lo[3], const double hi[3], const int 
     return CVR_ERR_CUDA;
   }
   cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, device);
-  if (dalloc(c, &c->flags, 6) != CVR_OK || dalloc(c, &c->counters, 2) != CVR_OK ||
+  if (cudaMallocHost(&c->back, sizeof(*c->back)) != cudaSuccess || dalloc(c, &c->flags, 6) != CVR_OK || dalloc(c, &c->counters, 2) != CVR_OK ||
       dalloc(c, &c->step_ctrl, SC_WORDS) != CVR_OK || dalloc(c, &c->step_part, 4 * (size_t)c->sms) != CVR_OK ||
       dalloc(c, &c->d_type_hist, MAX_TYPES + 1) != CVR_OK) {
     cudaEventDestroy(c->k_fork);
     cudaEventDestroy(c->k_join);
+    if (c->back) cudaFreeHost(c->back);
     cudaStreamDestroy(c->kstream);
     cudaStreamDestroy(c->stream);
     delete c;
@@ -1785,6 +1846,7 @@ void cvr_destroy(cvr_ctx *c) {
   cudaStreamSynchronize(c->stream);
   destroy_graphs(c);
   for (void *p : c->all_allocs) cudaFree(p);
+  cudaFreeHost(c->back);
   for (int k = 0; k < 2; ++k) {
     if (c->h_eta[k]) cudaFreeHost(c->h_eta[k]);
     if (c->eta_done[k]) cudaEventDestroy(c->eta_done[k]);
@@ -2059,19 +2121,15 @@ int cvr_set_state(cvr_ctx *c, int64_t n, const double *pos, const double *vel, c
     c->log2_tpa = (c->tpa == 32) ? 5 : (c->tpa == 8 ? 3 : 2);
   }
   // The types first, then the atoms per type on the GPU (the range check of
-  // every type, and the charge and mass sums at one term per type), read
-  // back with the positions behind them: the staged arrays reach the state
-  // only after the check.  The velocities follow on the side stream: on a
-  // context whose cells, tables and graphs stay, their copy runs beside the
-  // run's setup (list build and first forces, which need no velocities),
-  // done here, and they reach the atoms' places by id at the end.
+  // every type, and the charge and mass sums at one term per type): the
+  // staged arrays reach the state only if the check passes.  The velocities
+  // follow on the side stream and reach the atoms' places by id at the end.
   CVR_CUDA(c, cudaMemcpyAsync(c->stage_i, type, (size_t)n * sizeof(int32_t), cudaMemcpyHostToDevice, c->stream));
   CVR_CUDA(c, cudaMemsetAsync(c->d_type_hist, 0, (MAX_TYPES + 1) * sizeof(unsigned long long), c->stream));
   k_type_hist<<<std::min<int64_t>(grid_for(n, 256), 4 * 148), 256, 0, c->stream>>>(c->stage_i, (int)n, c->n_types,
                                                                                   c->d_type_hist);
   c->launches++;
-  unsigned long long per_type[MAX_TYPES + 1];
-  CVR_CUDA(c, cudaMemcpyAsync(per_type, c->d_type_hist, sizeof(per_type), cudaMemcpyDeviceToHost, c->stream));
+  const unsigned long long *bad = c->d_type_hist + MAX_TYPES;
   CVR_CUDA(c, cudaMemcpyAsync(c->stage, pos, (size_t)n * 3 * sizeof(double), cudaMemcpyHostToDevice, c->stream));
   if (mol) CVR_CUDA(c, cudaMemcpyAsync(c->stage_i + n, mol, (size_t)n * sizeof(int32_t), cudaMemcpyHostToDevice, c->stream));
   CVR_CUDA(c, cudaEventRecord(c->k_fork, c->stream));  // after the positions: they take the link first
@@ -2080,56 +2138,92 @@ int cvr_set_state(cvr_ctx *c, int64_t n, const double *pos, const double *vel, c
     CVR_CUDA(c, cudaMemcpyAsync(c->stage + 3 * n, vel, (size_t)n * 3 * sizeof(double), cudaMemcpyHostToDevice,
                                 c->kstream));
   CVR_CUDA(c, cudaEventRecord(c->k_join, c->kstream));
-  CVR_CUDA(c, cudaStreamSynchronize(c->stream));
-  if (per_type[MAX_TYPES] != 0) {
-    cudaStreamSynchronize(c->kstream);  // the caller's velocity array is borrowed until the copy ends
-    return fail(c, CVR_ERR_INVALID, "atom type out of range");
-  }
-  c->have_state = true;
   const bool mol_changed = (mol != nullptr) != c->use_mol;
-  c->use_mol = mol != nullptr;
-  double q2 = 0, mt = 0;
-  for (int t = 0; t < c->n_types; ++t) {
-    q2 += (double)per_type[t] * (c->charge[t] * c->charge[t]);
-    mt += (double)per_type[t] * c->mass[t];
+  // Same atom count and settings: cells, tables and buffers stay (and so do
+  // the step graphs).  The positions go to the state and the list is built,
+  // on the device gated by the type check, beside the velocity copy; one
+  // synchronisation at the end reads everything back.  (The slab correction's
+  // field depends on the force calls so far: there the first forces are done
+  // here too, as the next run's set-up.)
+  const bool kept = c->have_state && c->refreshed && !mol_changed && c->cap > 0 && !c->sc_on;
+  const int32_t *mol_d = mol ? c->stage_i + n : nullptr;
+  if (!kept) CVR_CUDA(c, cudaStreamSynchronize(c->stream));  // the checked upload first
+  const auto read_types = [&]() {
+    CVR_CUDA(c, cudaMemcpyAsync(c->back->per_type, c->d_type_hist, sizeof(c->back->per_type), cudaMemcpyDeviceToHost,
+                                c->stream));
+    return read_flags(c, c->back->flags);
+  };
+  if (!kept) {
+    if (int r = read_types()) return r;
+    if (c->back->per_type[MAX_TYPES] != 0) {
+      cudaStreamSynchronize(c->kstream);  // the caller's velocity array is borrowed until the copy ends
+      return fail(c, CVR_ERR_INVALID, "atom type out of range");
+    }
+    c->use_mol = mol != nullptr;
   }
-  // the step graphs bake these in (thermo kernel, pair-kernel choice)
-  if (mol_changed || mt != c->total_mass || q2 != c->q2_sum) c->epoch++;
-  c->total_mass = mt;
-  c->q2_sum = q2;
-  c->e_self = self_energy(c);
-  if (c->precision == CVR_PREC_FP64) {
-    DevState<double> s = dev_state<double>(c);
-    k_scatter_state<double><<<grid_for(n, 256), 256, 0, c->stream>>>(s, c->stage, nullptr, c->stage_i,
-                                                                      mol ? c->stage_i + n : nullptr);
-  } else {
-    DevState<float> s = dev_state<float>(c);
-    k_scatter_state<float><<<grid_for(n, 256), 256, 0, c->stream>>>(s, c->stage, nullptr, c->stage_i,
-                                                                    mol ? c->stage_i + n : nullptr);
-  }
+  if (c->precision == CVR_PREC_FP64)
+    k_scatter_state<double><<<grid_for(n, 256), 256, 0, c->stream>>>(dev_state<double>(c), c->stage, nullptr,
+                                                                      c->stage_i, mol_d, kept ? bad : nullptr);
+  else
+    k_scatter_state<float><<<grid_for(n, 256), 256, 0, c->stream>>>(dev_state<float>(c), c->stage, nullptr, c->stage_i,
+                                                                    mol_d, kept ? bad : nullptr);
   c->launches++;
-  CVR_CUDA(c, cudaMemsetAsync(c->flags, 0, 4 * sizeof(int), c->stream));
-  c->step = 0;
   int rs = CVR_OK;
-  if (!c->refreshed || mol_changed) {
-    rs = refresh(c);
+  if (kept) {
+    if (int r = DISPATCH(c, launch_build_now, c, 0)) return r;
   } else {
-    // same atom count and settings: cells, tables and buffers stay (and so
-    // do the step graphs); the list and the forces are redone now, beside
-    // the velocity copy (what the next run's setup would do)
+    CVR_CUDA(c, cudaMemsetAsync(c->flags, 0, 4 * sizeof(int), c->stream));
+    c->builds_seen = 0;
+  }
+  const auto sums = [&]() {
+    double q2 = 0, mt = 0;
+    for (int t = 0; t < c->n_types; ++t) {
+      q2 += (double)c->back->per_type[t] * (c->charge[t] * c->charge[t]);
+      mt += (double)c->back->per_type[t] * c->mass[t];
+    }
+    // the step graphs bake these in (thermo kernel, pair-kernel choice)
+    if (mol_changed || mt != c->total_mass || q2 != c->q2_sum) c->epoch++;
+    c->total_mass = mt;
+    c->q2_sum = q2;
+    c->e_self = self_energy(c);
+    c->have_state = true;
+    c->step = 0;
+    c->list_fresh = false;
     c->list_valid = false;
     c->setup_done = false;
-    rs = DISPATCH(c, setup_run, c);
+  };
+  if (!kept) {
+    sums();
+    rs = (!c->refreshed || mol_changed) ? refresh(c) : DISPATCH(c, setup_run, c);
   }
   // the host arrays are borrowed for this call only: the copies from them
   // (asynchronous when they are pinned) end before it returns
   cudaError_t e = cudaStreamWaitEvent(c->stream, c->k_join, 0);
   if (vel && e == cudaSuccess) {
     if (c->precision == CVR_PREC_FP64)
-      k_place_velocities<double><<<grid_for(n, 256), 256, 0, c->stream>>>(dev_state<double>(c), c->stage + 3 * n);
+      k_place_velocities<double><<<grid_for(n, 256), 256, 0, c->stream>>>(dev_state<double>(c), c->stage + 3 * n,
+                                                                          kept ? bad : nullptr);
     else
-      k_place_velocities<float><<<grid_for(n, 256), 256, 0, c->stream>>>(dev_state<float>(c), c->stage + 3 * n);
+      k_place_velocities<float><<<grid_for(n, 256), 256, 0, c->stream>>>(dev_state<float>(c), c->stage + 3 * n,
+                                                                         kept ? bad : nullptr);
     c->launches++;
+  }
+  if (kept && e == cudaSuccess) {
+    e = cudaMemsetAsync(c->flags, 0, sizeof(int), c->stream);  // the build is done
+    if (int r = read_types()) return r;
+    if (c->back->per_type[MAX_TYPES] != 0) return fail(c, CVR_ERR_INVALID, "atom type out of range");
+    sums();
+    int f = c->back->flags[1];
+    // a denser state than the list was sized for
+    for (int attempt = 0; (f & ERR_OVERFLOW) && attempt < 3; ++attempt) {
+      if (int r = regrow(c)) return r;
+      if (int r = DISPATCH(c, do_build, c, true)) return r;
+      CVR_CUDA(c, cudaMemsetAsync(c->flags, 0, sizeof(int), c->stream));
+      if (int r = read_flags(c, c->back->flags)) return r;
+      f = c->back->flags[1];
+    }
+    if (f & ERR_OVERFLOW) return fail(c, CVR_ERR_CAPACITY, "neighbour list overflow at setup");
+    c->list_valid = c->list_fresh = true;
   }
   const cudaError_t e2 = cudaStreamSynchronize(c->stream);
   if (e == cudaSuccess) e = e2;

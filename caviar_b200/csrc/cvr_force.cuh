@@ -1753,9 +1753,19 @@ __global__ void __launch_bounds__(256) k_type_hist(const int *__restrict__ type,
 
 template <typename real>
 __global__ void k_scatter_state(DevState<real> s, const double *__restrict__ pos, const double *__restrict__ vel,
-                                const int *__restrict__ typ, const int *__restrict__ mol) {
+                                const int *__restrict__ typ, const int *__restrict__ mol,
+                                const unsigned long long *__restrict__ bad) {
+  // bad (nullable): types out of range; then the state stays as it was and
+  // the rebuild flag, which this kernel otherwise raises, gates what follows
+  if (bad && *bad) return;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= s.n) return;
+  if (bad && i == 0) {
+    *s.flag = 1;
+    *s.err = 0;
+    *s.max_count = 0;
+    *s.n_builds = 0;
+  }
   s.x[i] = pos[3 * (size_t)i];
   s.y[i] = pos[3 * (size_t)i + 1];
   s.z[i] = pos[3 * (size_t)i + 2];
@@ -1773,13 +1783,34 @@ __global__ void k_scatter_state(DevState<real> s, const double *__restrict__ pos
 // Velocities in the caller's order (AoS) to the atoms' current places, by
 // id: the state may have been reordered since the positions were placed.
 template <typename real>
-__global__ void k_place_velocities(DevState<real> s, const double *__restrict__ vel) {
+__global__ void k_place_velocities(DevState<real> s, const double *__restrict__ vel,
+                                   const unsigned long long *__restrict__ bad) {
+  if (bad && *bad) return;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= s.n) return;
   const size_t k = 3 * (size_t)s.id[i];
   s.vx[i] = vel[k];
   s.vy[i] = vel[k + 1];
   s.vz[i] = vel[k + 2];
+}
+
+// Arrays copied in one launch (one block column each), 16 bytes at a time
+// and a tail of bytes.
+constexpr int COPY_MAX = 20;
+struct CopyArgs {
+  const void *src[COPY_MAX];
+  void *dst[COPY_MAX];
+  size_t bytes[COPY_MAX];
+};
+__global__ void __launch_bounds__(256) k_copy_arrays(CopyArgs a) {
+  const int q = blockIdx.y;
+  const size_t n = a.bytes[q], words = n / 16;
+  const uint4 *src = static_cast<const uint4 *>(a.src[q]);
+  uint4 *dst = static_cast<uint4 *>(a.dst[q]);
+  const size_t stride = (size_t)gridDim.x * blockDim.x, t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  for (size_t i = t; i < words; i += stride) dst[i] = src[i];
+  const size_t rest = words * 16 + t;
+  if (rest < n) static_cast<char *>(a.dst[q])[rest] = static_cast<const char *>(a.src[q])[rest];
 }
 
 }  // namespace cvr

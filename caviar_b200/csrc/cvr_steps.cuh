@@ -158,6 +158,14 @@ __device__ __forceinline__ void scan_cells(const int *count, int *start, int nce
   if (c1 == ncells && c0 < c1 && threadIdx.x == 0) start[ncells] = before;
 }
 
+// One warp's list-search pieces inside the block's dynamic shared memory.
+__device__ __forceinline__ WarpPieces warp_pieces(unsigned char *sm, int warp, int warps) {
+  float4 *geo = reinterpret_cast<float4 *>(sm);
+  int *off = reinterpret_cast<int *>(geo + warps * PIECES_MAX);
+  uint32_t *pc = reinterpret_cast<uint32_t *>(off + warps * (PIECES_MAX + 1));
+  return WarpPieces{off + warp * (PIECES_MAX + 1), geo + warp * PIECES_MAX, pc + warp * PIECES_MAX};
+}
+
 // Block-wide sum of NV doubles into out[0..NV) (fixed order).
 template <int NV>
 __device__ __forceinline__ void block_sum_to(double (&v)[NV], double *out) {
@@ -197,12 +205,7 @@ __global__ void __launch_bounds__(STEP_THREADS, 1) k_steps(DevState<real> s, Ste
   grid.init(a.ctrl + 2 * a.launch);
   const Stencil<real> st = stencil_of(s);
   const EwrArgs<real> no_ewald{};
-  constexpr int pieces = PIECES_MAX;
-  WarpPieces wp;
-  wp.geo = reinterpret_cast<float4 *>(smraw) + warp * pieces;
-  wp.off = reinterpret_cast<int *>(reinterpret_cast<float4 *>(smraw) + WARPS * pieces) + warp * (pieces + 1);
-  wp.pc = reinterpret_cast<uint32_t *>(reinterpret_cast<int *>(reinterpret_cast<float4 *>(smraw) + WARPS * pieces) +
-                                       WARPS * (pieces + 1)) + warp * pieces;
+  const WarpPieces wp = warp_pieces(smraw, warp, WARPS);
   real4 *buf[2] = {s.x4, a.x4b};
   DevState<real> built = s;  // as the list search sees it
   built.x = a.bx;
@@ -459,6 +462,42 @@ __global__ void __launch_bounds__(STEP_THREADS, 1) k_steps(DevState<real> s, Ste
       a.ts.scal[1] = zeta;
     }
   }
+}
+
+// A forced list build (count_only: the neighbour counts alone) in one launch
+// for the systems k_steps takes: the stages of launch_build between grid
+// barriers.  Eight launches of 2-4 us each and their gaps otherwise.  Returns
+// at once if the rebuild flag is not set.
+template <typename real>
+__global__ void __launch_bounds__(STEP_THREADS, 1)
+    k_build_once(DevState<real> s, unsigned long long *ctrl, int launch, int count_only, int log2_tpa) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  __shared__ GridBarrier grid;
+  __shared__ int red[STEP_THREADS / 32];
+  const int n = s.n, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  const int tid = blockIdx.x * blockDim.x + threadIdx.x, nthreads = gridDim.x * blockDim.x;
+  if (tid < 2) ctrl[2 * (launch ^ 1) + tid] = 0;
+  if (*s.flag == 0) return;
+  grid.init(ctrl + 2 * launch);
+  for (int i = tid; i < n; i += nthreads) bin_atom(s, i);
+  if (grid.meet(s.err) & 2) return;
+  if (tid == 0) {
+    *s.build_epoch += 1;
+    if (!count_only) atomicAdd(s.n_builds, 1);
+  }
+  scan_cells(s.cell_count, s.cell_start, s.cells.ncells, red);
+  if (grid.meet(s.err) & 2) return;
+  for (int i = tid; i < n; i += nthreads) scatter_atom(s, i);
+  if (grid.meet(s.err) & 2) return;
+  for (int c = tid; c < s.cells.ncells; c += nthreads) s.cell_count[c] = s.cell_fill[c] = 0;
+  for (int t = tid; t < n; t += nthreads) {
+    const int i = s.slot_atom[t];
+    place_atom(s, place_of(s, i), i, s.x4);
+  }
+  if (grid.meet(s.err) & 2) return;
+  const WarpPieces wp = warp_pieces(smraw, warp, warps);
+  for (int i = blockIdx.x * warps + warp; i < n; i += gridDim.x * warps)
+    list_search_warp(s, i, lane, wp, count_only, log2_tpa);
 }
 
 // one record's sums for n atoms (at most one k_pair warp per atom)
