@@ -8,8 +8,9 @@
 // exchange_ghost_single_md_domain.cpp:59-99).  Physics per replica: LJ with
 // the reference's linear force shift (lj.cpp:439-448) up to rc_lj, Ewald real
 // space (electrostatic_ewald_r.cpp:196-198) up to rc_r <= L/2 under the
-// minimum image (all pairs: at rc = L/2 half of all pairs are inside, so a
-// cell list would save at most 2x), Ewald k space over the reference's k-set
+// minimum image (all charged pairs: at rc = L/2 half of them are inside, so a
+// cell list would save at most 2x; LJ from a pair list in all but the
+// smallest replicas), Ewald k space over the reference's k-set
 // (initialize.cpp:184-222) and force (electrostatic_ewald_k.cpp:197-234).
 //
 // Layout: FP64 positions/velocities in global memory (concatenated, SoA);
@@ -58,6 +59,16 @@ struct KRunB {
   int nx, ny, nz0, len, k0, skip;
 };
 
+// LJ pair lists of the larger replicas: entries per atom, skin as a fraction
+// of the LJ cutoff, and the smallest replica that uses one.  With all pairs,
+// three tiles in four hold no charged pair and test 32 x 32 atoms for the few
+// per cent within the LJ cutoff.  50 steps of 296 equal replicas, all pairs ->
+// list: 5.51 -> 5.67 ms at 150 atoms, 7.20 -> 6.53 at 200, 12.4 -> 11.5 at 400,
+// 24.6 -> 19.0 at 600; 1024 replicas of 64-2048 atoms, 20 steps: 83.7 -> 57.5 ms.
+constexpr int LCAP = 128;
+constexpr double LSKIN = 0.12;
+constexpr int LIST_MIN = 192;
+
 constexpr int KFILL_MASK = (1 << 30) - 1;
 constexpr int KTWICE = 1 << 30;
 
@@ -75,6 +86,12 @@ struct BatchDev {
   // filled from it), bit 30 = k's force term counts twice (its mirror is skipped)
   const int *kinfo;
   double *out;  // [replica][NTH]
+  // LJ lists: of replica r, entry k of atom i at list[LCAP * off[r] + k * n + i];
+  // neighbours per atom; coordinates at the build, SoA [3][atoms]
+  uint16_t *list;
+  int *list_count;
+  uint32_t *list_u;
+  long long n_total;
   int nk, nruns, kmax, n_types;
   float eps[TMAX * TMAX], sig[TMAX * TMAX], charge[TMAX];
   double mass[TMAX], mass_inv[TMAX], chargeD[TMAX];
@@ -172,7 +189,7 @@ struct PairK {
 
 // One ordered pair (i, j): c with F_i += c d, d = r_j - r_i (minimum image).
 // EWR: this pair may carry charge on both ends.  Energies into e[0..2] (lj, ewr, virial) scaled by w.
-template <bool UNI, bool EWR, bool EV>
+template <bool UNI, bool EWR, bool EV, bool LJ = true>
 __device__ __forceinline__ float pair_c(const Smem &S, const PairK &K, const float4 &ih, const float4 &il,
                                         const float4 &jh, const float4 &jl, float (&d)[3], double (&e)[3], double w) {
   // minimum image: the wrapping difference of the fixed-point coordinates
@@ -190,7 +207,7 @@ __device__ __forceinline__ float pair_c(const Smem &S, const PairK &K, const flo
     le = S.lje[tp];
   }
   float c = 0.f;
-  if (r2 <= K.rc2 && lc.y != 0.f) {
+  if (LJ && r2 <= K.rc2 && lc.y != 0.f) {
     const float r2i = __fdividef(1.f, r2), s2 = lc.x * r2i, s6 = s2 * s2 * s2;
     c = r2i * s6 * (lc.y - lc.z * s6) + lc.w;
     if (EV) e[0] += w * (double)(le.x * (s6 * s6 - s6) + le.z * r2 + le.y);
@@ -213,7 +230,7 @@ __device__ __forceinline__ float pair_c(const Smem &S, const PairK &K, const flo
 // each unordered pair once (Newton's third law).  Lane l meets atom
 // J*32 + (l + s) % 32 at step s; the reaction force on that atom travels with
 // it (shuffled one lane down per step) and is home after 32 steps.
-template <bool UNI, bool EWR, bool EV>
+template <bool UNI, bool EWR, bool EV, bool LJ>
 __device__ __forceinline__ void tile(const Smem &S, const PairK &K, int I, int J, int n, double (&e)[3]) {
   const int lane = threadIdx.x & 31;
   const int i = I * 32 + lane;
@@ -226,7 +243,7 @@ __device__ __forceinline__ void tile(const Smem &S, const PairK &K, int I, int J
     if (vi && j < n) {
       const float4 jh = S.xh[j], jl = S.xl[j];
       float d[3];
-      const float c = pair_c<UNI, EWR, EV>(S, K, ih, il, jh, jl, d, e, 1.0);
+      const float c = pair_c<UNI, EWR, EV, LJ>(S, K, ih, il, jh, jl, d, e, 1.0);
 #pragma unroll
       for (int a = 0; a < 3; ++a) {
         fi[a] = fmaf(c, d[a], fi[a]);
@@ -246,7 +263,7 @@ __device__ __forceinline__ void tile(const Smem &S, const PairK &K, int I, int J
 }
 
 // Diagonal tile: ordered pairs inside block I (each pair from both ends).
-template <bool UNI, bool EWR, bool EV>
+template <bool UNI, bool EWR, bool EV, bool LJ>
 __device__ __forceinline__ void tile_diag(const Smem &S, const PairK &K, int I, int n, double (&e)[3]) {
   const int lane = threadIdx.x & 31;
   const int i = I * 32 + lane;
@@ -258,7 +275,7 @@ __device__ __forceinline__ void tile_diag(const Smem &S, const PairK &K, int I, 
     if (vi && j < n) {
       const float4 jh = S.xh[j], jl = S.xl[j];
       float d[3];
-      const float c = pair_c<UNI, EWR, EV>(S, K, ih, il, jh, jl, d, e, 0.5);
+      const float c = pair_c<UNI, EWR, EV, LJ>(S, K, ih, il, jh, jl, d, e, 0.5);
 #pragma unroll
       for (int a = 0; a < 3; ++a) fi[a] = fmaf(c, d[a], fi[a]);
     }
@@ -268,11 +285,75 @@ __device__ __forceinline__ void tile_diag(const Smem &S, const PairK &K, int I, 
   S.fsz[i] += fi[2];
 }
 
+// The LJ list of the current positions: every pair within the LJ cutoff plus
+// the skin, in both atoms' rows, partners in ascending order (so a row's
+// terms are summed in the same order whenever the list was built).  False
+// (for the whole block) if a row overflows.  Each thread searches for its own
+// atoms, all lanes of a warp reading the same partner.  The test runs on the
+// displacements' top 15 bits in integers (units of L / 2^15, each axis off by
+// less than one; rl2 is widened for that): converting three differences to
+// float would keep the conversion unit busy for twice the test's issue slots.
+template <int TPB>
+__device__ bool build_lj_list(const BatchDev &p, const Smem &S, int n, long long o, int rl2) {
+  uint16_t *list = p.list + (size_t)LCAP * o;
+  bool over = false;
+  for (int i = threadIdx.x; i < n; i += TPB) {
+    const float4 ih = S.xh[i];
+    const uint32_t ux = __float_as_uint(ih.x), uy = __float_as_uint(ih.y), uz = __float_as_uint(ih.z);
+    int cnt = 0;
+#pragma unroll 4
+    for (int j = 0; j < n; ++j) {
+      const float4 jh = S.xh[j];
+      const int dx = (int)(__float_as_uint(jh.x) - ux) >> 17, dy = (int)(__float_as_uint(jh.y) - uy) >> 17,
+                dz = (int)(__float_as_uint(jh.z) - uz) >> 17;
+      if (dx * dx + dy * dy + dz * dz <= rl2 && j != i) {
+        if (cnt < LCAP) list[(size_t)cnt * n + i] = (uint16_t)j;
+        ++cnt;
+      }
+    }
+    over = over || cnt > LCAP;
+    p.list_count[o + i] = min(cnt, LCAP);
+    p.list_u[o + i] = ux;
+    p.list_u[p.n_total + o + i] = uy;
+    p.list_u[2 * p.n_total + o + i] = uz;
+  }
+  return !__syncthreads_or(over);
+}
+
+// LJ forces from the list, each thread its own atoms, added to S.fs* (units
+// of h); energies and virial into e as pair_c (both ends: weight 1/2).
+template <int TPB, bool UNI, bool EV>
+__device__ __forceinline__ void lj_list(const BatchDev &p, const Smem &S, const PairK &K, int n, long long o,
+                                        double (&e)[3]) {
+  for (int i = threadIdx.x; i < n; i += TPB) {
+    const float4 ih = S.xh[i], none = make_float4(0.f, 0.f, 0.f, 0.f);
+    const uint16_t *row = p.list + (size_t)LCAP * o + i;
+    const int cnt = p.list_count[o + i];
+    float f[3] = {0.f, 0.f, 0.f};
+    for (int k = 0; k < cnt; k += 4) {
+      int j[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) j[u] = k + u < cnt ? (int)row[(size_t)(k + u) * n] : -1;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        if (j[u] < 0) continue;
+        float d[3];
+        const float c = pair_c<UNI, false, EV>(S, K, ih, none, S.xh[j[u]], none, d, e, 0.5);
+#pragma unroll
+        for (int a = 0; a < 3; ++a) f[a] = fmaf(c, d[a], f[a]);
+      }
+    }
+    S.fsx[i] += f[0];
+    S.fsy[i] += f[1];
+    S.fsz[i] += f[2];
+  }
+}
+
 // Forces of the replica's current positions into S.fs* (all pairs under the
 // minimum image, then k space).  EV: energies and virial into ev[0..4]
 // (this thread's share: lj, ewald_r, ewald_k, -, virial).
 template <int TPB, bool UNI, bool EV>
-__device__ void batch_forces(const BatchDev &p, const Smem &S, int r, int n, int nq, double L, int G,
+__device__ void batch_forces(const BatchDev &p, const Smem &S, int r, int n, int nq, double L, int G, bool listed,
                              double (&ev)[5]) {
   constexpr int W = TPB / 32;
   const int warp = threadIdx.x >> 5;
@@ -286,12 +367,14 @@ __device__ void batch_forces(const BatchDev &p, const Smem &S, int r, int n, int
   K.ke = (float)(p.k_e / h);
   K.lc = S.ljc[0];
   K.le = S.lje[0];
-  const int nb = (n + 31) >> 5;
-  for (int i = threadIdx.x; i < nb * 32; i += TPB) S.fsx[i] = S.fsy[i] = S.fsz[i] = 0.f;
+  const int all = (n + 31) & ~31;
+  for (int i = threadIdx.x; i < all; i += TPB) S.fsx[i] = S.fsy[i] = S.fsz[i] = 0.f;
   __syncthreads();
   double e[3] = {0, 0, 0};
   // ---- pairs: round-robin schedule of block pairs (circle method), every
-  // block in at most one tile per round, a barrier between rounds
+  // block in at most one tile per round, a barrier between rounds.  With an
+  // LJ list (listed) only the blocks of charged atoms meet, for Ewald alone.
+  const int nb = listed ? (nq + 31) >> 5 : all >> 5;
   const int nbe = nb + (nb & 1), m = nbe - 1, half = nbe >> 1;
   for (int round = 0; round < m; ++round) {
     for (int q = warp; q < half; q += W) {
@@ -305,24 +388,32 @@ __device__ void batch_forces(const BatchDev &p, const Smem &S, int r, int n, int
       }
       if (I >= nb || J >= nb) continue;
       const bool ewr = (I * 32 < nq) && (J * 32 < nq);  // warp-uniform: charged atoms come first
-      if (ewr)
-        tile<UNI, true, EV>(S, K, I, J, n, e);
+      if (listed)
+        tile<UNI, true, EV, false>(S, K, I, J, n, e);
+      else if (ewr)
+        tile<UNI, true, EV, true>(S, K, I, J, n, e);
       else
-        tile<UNI, false, EV>(S, K, I, J, n, e);
+        tile<UNI, false, EV, true>(S, K, I, J, n, e);
     }
     __syncthreads();
   }
   for (int I = warp; I < nb; I += W) {
-    if (I * 32 < nq)
-      tile_diag<UNI, true, EV>(S, K, I, n, e);
+    if (listed)
+      tile_diag<UNI, true, EV, false>(S, K, I, n, e);
+    else if (I * 32 < nq)
+      tile_diag<UNI, true, EV, true>(S, K, I, n, e);
     else
-      tile_diag<UNI, false, EV>(S, K, I, n, e);
+      tile_diag<UNI, false, EV, true>(S, K, I, n, e);
   }
   __syncthreads();
+  if (listed) {
+    lj_list<TPB, UNI, EV>(p, S, K, n, p.off[r], e);
+    __syncthreads();
+  }
   // pair forces from units of h back to length units
   {
     const float inv_h = (float)(4294967296.0 / L);
-    for (int i = threadIdx.x; i < nb * 32; i += TPB) {
+    for (int i = threadIdx.x; i < all; i += TPB) {
       S.fsx[i] *= inv_h;
       S.fsy[i] *= inv_h;
       S.fsz[i] *= inv_h;
@@ -516,9 +607,23 @@ __global__ void __launch_bounds__(TPB, 1) k_batch(BatchDev p, int first, int nst
     }
   }
   __syncthreads();
+  // the LJ list (larger replicas): rebuilt when an atom has moved half the
+  // skin since the build (a little less, for the rounding of the test)
+  const bool wants_list = n >= LIST_MIN;
+  int rl2 = 0;
+  float moved2 = 0.f;
+  bool listed = false;
+  if (wants_list) {
+    // below (0.56 x 2^15 + 1.8)^2 < 2^31: the cutoff is at most half the box
+    const double rl = p.rc_lj[r] * (1.0 + LSKIN) * 32768.0 / L + 1.7320508075688774;
+    const double half = 0.4999 * p.rc_lj[r] * LSKIN * 4294967296.0 / L;
+    rl2 = (int)ceil(rl * rl);
+    moved2 = (float)(half * half);
+    listed = build_lj_list<TPB>(p, S, n, o, rl2);
+  }
   double ev[5] = {0, 0, 0, 0, 0};
   if (compute_first) {
-    batch_forces<TPB, UNI, false>(p, S, r, n, nq, L, G, ev);
+    batch_forces<TPB, UNI, false>(p, S, r, n, nq, L, G, listed, ev);
   } else {
     for (int i = threadIdx.x; i < n; i += TPB) {
       S.fsx[i] = p.fx[o + i];
@@ -529,6 +634,7 @@ __global__ void __launch_bounds__(TPB, 1) k_batch(BatchDev p, int first, int nst
   const double dt = p.dt, h = 0.5 * dt;
   for (int step = 0; step < nsteps; ++step) {
     __syncthreads();
+    bool moved = false;
     for (int i = threadIdx.x; i < n; i += TPB) {
       const long long gi = o + i;
       const double mi = p.mass_inv[p.type[gi]];
@@ -543,9 +649,16 @@ __global__ void __launch_bounds__(TPB, 1) k_batch(BatchDev p, int first, int nst
         X[a][gi] = x;
       }
       to_smem(p, S, i, gi, L);
+      if (wants_list) {
+        const float4 u = S.xh[i];
+        const float dx = (float)(int)(__float_as_uint(u.x) - p.list_u[gi]),
+                    dy = (float)(int)(__float_as_uint(u.y) - p.list_u[p.n_total + gi]),
+                    dz = (float)(int)(__float_as_uint(u.z) - p.list_u[2 * p.n_total + gi]);
+        moved = moved || !(dx * dx + dy * dy + dz * dz <= moved2);
+      }
     }
-    __syncthreads();
-    batch_forces<TPB, UNI, false>(p, S, r, n, nq, L, G, ev);
+    if (__syncthreads_or(moved)) listed = build_lj_list<TPB>(p, S, n, o, rl2);
+    batch_forces<TPB, UNI, false>(p, S, r, n, nq, L, G, listed, ev);
     for (int i = threadIdx.x; i < n; i += TPB) {
       const long long gi = o + i;
       const double mi = p.mass_inv[p.type[gi]];
@@ -561,7 +674,7 @@ __global__ void __launch_bounds__(TPB, 1) k_batch(BatchDev p, int first, int nst
     p.fz[o + i] = S.fsz[i];
   }
   __syncthreads();
-  batch_forces<TPB, UNI, true>(p, S, r, n, nq, L, G, ev);  // energies only; S.fs* is scratch here
+  batch_forces<TPB, UNI, true>(p, S, r, n, nq, L, G, listed, ev);  // energies only; S.fs* is scratch here
   __syncthreads();
   // kinetic energy (COM removed), energies
   double kv[9] = {0, 0, 0, 0, 0, ev[0], ev[1], ev[4], ev[2]};
@@ -821,6 +934,11 @@ int cvr_batch_create(cvr_batch **out, int n_rep, const int64_t *n_atoms, const d
   d.vz = arr + 5 * N;
   cudaMemset(farr, 0, 3 * N * sizeof(float));
   cudaMemset(dtype, 0, N * sizeof(int));
+  uint16_t *list;
+  if ((rc = balloc(b, &list, (size_t)LCAP * N)) || (rc = balloc(b, &d.list_count, N)) || (rc = balloc(b, &d.list_u, 3 * N)))
+    return rc;
+  d.list = list;
+  d.n_total = o;
   d.fx = farr;
   d.fy = farr + N;
   d.fz = farr + 2 * N;
