@@ -410,7 +410,7 @@ __global__ void __launch_bounds__(KRED_E *KRED_G) k_adj_kreduce(Params p, const 
 
 // FP32 (mixed) pair terms use the hardware reciprocal / reciprocal square
 // root / exponential and erfc from Abramowitz & Stegun 7.1.26 sharing the
-// Gaussian (erfc_as); the FP64 form keeps the correctly rounded functions.
+// Gaussian (erfc_as); FP64 takes the library's functions and erfc_ex.
 __device__ __forceinline__ float adj_rcp(float x) { return __fdividef(1.f, x); }
 __device__ __forceinline__ double adj_rcp(double x) { return 1.0 / x; }
 
@@ -541,7 +541,7 @@ __global__ void __launch_bounds__(PAIR_WARPS * 32, sizeof(real) == 4 ? 4 : 2)
           r = sqrt(r2);
           ri = (real)1 / r;
           G = exp(-pc.alpha2 * r2);
-          ec = erfc(pc.alpha * r);
+          ec = cvr::erfc_ex(pc.alpha * r, G);
         }
         const real E1 = -pc.beta * G * ri - ec * ri * ri, cq = pc.ke * E1 * ri;
         real c1 = (real)0;

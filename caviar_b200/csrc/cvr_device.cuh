@@ -112,6 +112,46 @@ __device__ __forceinline__ float erfc_as(float x, float ex) {
                   0.254829592f) * ex;
 }
 
+// erfc(x) for x >= 0 in FP64 from ex = exp(-x^2), which the Ewald real-space
+// force needs anyway: (1 + 2x) exp(x^2) erfc(x) as a polynomial in
+// t = (x - 3.75) / (x + 3.75) (M. M. Shepherd and J. G. Laframboise, Math.
+// Comp. 36 (1981) 249).  The 23 coefficients are the Chebyshev interpolant of
+// degree 22 at 300 nodes, computed at 60 digits and expanded in powers of t;
+// exp(x^2) erfc(x) comes out within 6.5e-16 relative on [0, 12].  Even and odd
+// powers in two chains, no branches: the four pairs a lane has in flight
+// interleave, which the library function's branches prevent.  8000 ions, pair
+// kernel alone: 76.4 us with the library's erfc (FP64 pipe 43 % busy), 56.5
+// with this; trajectory adjoint at 1372 atoms 38.8 -> 34.0.
+__device__ __forceinline__ double erfc_ex(double x, double ex) {
+  const double a = x + 3.75, b = fma(2.0, x, 1.0);
+  const double r = 1.0 / (a * b);
+  const double t = (x - 3.75) * b * r, u = t * t;
+  double p = -2.6231073471334759e-09;
+  p = fma(p, u, 3.1979266716668042e-08);
+  p = fma(p, u, -2.4857126248016745e-07);
+  p = fma(p, u, 1.7419821586224816e-06);
+  p = fma(p, u, -1.1438048033346894e-05);
+  p = fma(p, u, 5.1646529741774162e-05);
+  p = fma(p, u, 0.00029371437804495801);
+  p = fma(p, u, -0.0097465796832652621);
+  p = fma(p, u, -0.05869339857664934);
+  p = fma(p, u, -0.10880393014244462);
+  p = fma(p, u, 0.0035854154854790257);
+  p = fma(p, u, 1.2375126308378275);
+  double q = -1.9551358868985616e-09;
+  q = fma(q, u, 1.8790823223700481e-08);
+  q = fma(q, u, -5.0844653786873023e-08);
+  q = fma(q, u, -9.7926257073035231e-07);
+  q = fma(q, u, 2.2387565714911816e-05);
+  q = fma(q, u, -0.00029015535246077655);
+  q = fma(q, u, 0.0017556261651970652);
+  q = fma(q, u, 0.028362277372111139);
+  q = fma(q, u, 0.09230432116428125);
+  q = fma(q, u, 0.08227673848999506);
+  q = fma(q, u, -0.14024059858554525);
+  return fma(q, t, p) * (a * r) * ex;
+}
+
 // 32-bit fixed-point coordinate u = round(p * 2^32 / L) mod 2^32.  The
 // difference of two such coordinates, read as a signed int32, is the
 // minimum-image displacement in units of L / 2^32 whenever the true

@@ -48,7 +48,6 @@ __device__ __forceinline__ float fast_rsqrt(float x) { return rsqrtf(x); }
 __device__ __forceinline__ double fast_rsqrt(double x) { return rsqrt(x); }
 __device__ __forceinline__ float fast_exp(float x) { return __expf(x); }
 __device__ __forceinline__ double fast_exp(double x) { return exp(x); }
-__device__ __forceinline__ double erfc_r(double x) { return erfc(x); }
 __device__ __forceinline__ int type_of(float w) { return __float_as_int(w); }
 __device__ __forceinline__ int type_of(double w) { return (int)w; }
 __device__ __forceinline__ void sincospi_r(float a, float *s, float *c) { sincospif(a, s, c); }
@@ -174,7 +173,7 @@ __device__ __forceinline__ void pair_term(PairAcc<real> &A, real dx, real dy, re
       if constexpr (sizeof(real) == 4)
         erfcv = erfc_as(ew.alpha * r, ex);  // shares ex with the force term
       else
-        erfcv = erfc_r(ew.alpha * r);
+        erfcv = erfc_ex(ew.alpha * r, ex);
       const real sv = (ew.two_alpha_spi * ex + erfcv * rinv) * (rinv * rinv);
       const real lam = same_mol ? pc.lam : (real)1;
       c -= lam * pc.qq * sv;
