@@ -199,6 +199,7 @@ struct cvr_ctx {
   unsigned long long *step_ctrl{};
   double *step_part{}, *step_rec{}, *step_pos{};
   int step_launch = 0;
+  int64_t steps_n = 0;  // atoms the buffers are sized for
   // Langevin integrator (md_simulator.cpp:670-811)
   int integrator = 0;  // 0 velocity Verlet, 1 velocity Verlet Langevin
   double lgv_temperature = -1, lgv_friction = 0, lgv_kb = -1, lgv_kbt = -1;
@@ -629,10 +630,7 @@ int alloc_atoms(cvr_ctx *c, int64_t n) {
   if ((r = dalloc(c, (unsigned char **)&c->ay, n * rs))) return r;
   if ((r = dalloc(c, (unsigned char **)&c->az, n * rs))) return r;
   if ((r = dalloc(c, (unsigned char **)&c->x4, n * 4 * rs))) return r;
-  const size_t ns = n <= STEPS_MAX_ATOMS ? n : 0;  // the buffers of k_steps
-  if ((r = dalloc(c, (unsigned char **)&c->x4b, ns * 4 * rs))) return r;
-  if ((r = dalloc(c, &c->step_rec, 2 * steps_record_doubles(ns)))) return r;
-  if ((r = dalloc(c, &c->step_pos, 3 * ns))) return r;
+  c->steps_n = 0;
   // per-atom arrays that a replay after a list overflow restores
   c->snap_pairs.clear();
   c->snap_bytes.clear();
@@ -1343,6 +1341,12 @@ bool steps_in_one(const cvr_ctx *c) {
 template <typename real, int TPA, bool ONE_TYPE, bool FIXED>
 int launch_steps_t(cvr_ctx *c, int nsteps, int64_t every, int64_t done) {
   const GridShape g = grid_shape(c, grid_for(c->n, 32 / TPA));
+  if (c->steps_n != c->n) {
+    if (int r = dalloc(c, (unsigned char **)&c->x4b, c->n * 4 * sizeof(real))) return r;
+    if (int r = dalloc(c, &c->step_rec, 2 * steps_record_doubles(c->n))) return r;
+    if (int r = dalloc(c, &c->step_pos, 3 * (size_t)c->n)) return r;
+    c->steps_n = c->n;
+  }
   const double h = FIXED ? c->L[0] / std::ldexp(1.0, 32) : 1.0;  // as launch_pair_t
   StepArgs<real> a{};
   a.coef = (const PairCoef<real> *)c->d_coef;
