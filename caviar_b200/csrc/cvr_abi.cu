@@ -622,7 +622,7 @@ int alloc_atoms(cvr_ctx *c, int64_t n) {
   if ((r = dalloc(c, &c->ptr, (cnt)))) return r;
   A(x, n) A(y, n) A(z, n) A(vx, n) A(vy, n) A(vz, n);
   A(tx, n) A(ty, n) A(tz, n) A(tvx, n) A(tvy, n) A(tvz, n);
-  A(xb, n) A(cell, n) A(id, n) A(type, n) A(mol, n) A(gcls, n);
+  A(xb, n + CVR_BUILD_UNROLL) A(cell, n) A(id, n) A(type, n) A(mol, n) A(gcls, n);
   A(tid, n) A(ttype, n) A(tmol, n) A(tcell, n) A(slot_atom, n) A(perm, n);
   A(ncount, n) A(stage, 6 * n) A(stage_i, 2 * n);
 #undef A
