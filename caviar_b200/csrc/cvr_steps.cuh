@@ -392,12 +392,12 @@ __global__ void __launch_bounds__(STEP_THREADS, 1) k_steps(DevState<real> s, Ste
     if (two_pass) {
       if (grid.meet(s.err) & 2) return;
       if (ts) {
-        if (warp < 4) {  // every block sums the partials in the same order
+        for (int q = warp; q < 4; q += WARPS) {  // every block sums the partials in the same order
           double x = 0.0;
-          for (int b = lane; b < (int)gridDim.x; b += 32) x += a.part[4 * b + warp];
+          for (int b = lane; b < (int)gridDim.x; b += 32) x += a.part[4 * b + q];
 #pragma unroll
           for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-          if (lane == 0) ke_sum[warp] = x;
+          if (lane == 0) ke_sum[q] = x;
         }
         __syncthreads();
         const double sums[4] = {ke_sum[0], ke_sum[1], ke_sum[2], ke_sum[3]};
