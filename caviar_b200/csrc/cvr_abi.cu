@@ -1464,15 +1464,23 @@ int build_graphs(cvr_ctx *c) {
   return CVR_OK;
 }
 
+// The first forces of a state whose list cvr_set_state built (the caller
+// reads the flags).
 template <typename real>
-int run_impl(cvr_ctx *c, int64_t nsteps, int64_t every, double *thermo) {
-  if (!c->setup_done && c->list_fresh) {
-    if (int r = forces_now<real>(c, false)) return r;  // its errors are read with the run's
+int fresh_forces(cvr_ctx *c) {
+  if (c->list_fresh && !c->setup_done) {
+    if (int r = forces_now<real>(c, false)) return r;
     c->setup_done = true;
-  } else if (!c->setup_done) {
-    if (int r = setup_run<real>(c)) return r;
   }
   c->list_fresh = false;
+  return CVR_OK;
+}
+
+template <typename real>
+int run_impl(cvr_ctx *c, int64_t nsteps, int64_t every, double *thermo) {
+  if (int r = fresh_forces<real>(c)) return r;  // its errors are read with the run's
+  if (!c->setup_done)
+    if (int r = setup_run<real>(c)) return r;
   const int64_t nrec = (every > 0) ? nsteps / every : 0;
   if ((size_t)nrec > c->thermo_cap) {
     if (int r = dalloc(c, &c->d_thermo, (size_t)std::max<int64_t>(nrec, 1) * CVR_N_THERMO)) return r;
@@ -1786,6 +1794,17 @@ int pairs_impl(cvr_ctx *c, std::vector<std::array<int32_t, 5>> &out) {
 }  // namespace
 
 #define DISPATCH(c, fn, ...) ((c)->precision == CVR_PREC_FP64 ? fn<double>(__VA_ARGS__) : fn<float>(__VA_ARGS__))
+
+namespace {
+// What a caller reads back (accelerations, S(k)) belongs to the state set last.
+int current_forces(cvr_ctx *c) {
+  if (!c->list_fresh || c->setup_done) return CVR_OK;
+  if (int r = DISPATCH(c, fresh_forces, c)) return r;
+  if (int r = read_flags(c, c->back->flags)) return r;
+  if (c->back->flags[1] & ERR_KSPACE_TC) return fail(c, CVR_ERR_CUDA, "tensor-core k-space force: a wait ran out");
+  return CVR_OK;
+}
+}  // namespace
 
 extern "C" {
 
@@ -2288,6 +2307,8 @@ int cvr_get_state(cvr_ctx *c, double *pos, double *vel, double *acc) {
   if (!c) return CVR_ERR_INVALID;
   if (!c->have_state) return fail(c, CVR_ERR_STATE, "no state");
   cudaSetDevice(c->device);
+  if (acc)
+    if (int r = current_forces(c)) return r;
   const int64_t n = c->n;
   double *dp = c->stage, *dv = c->stage + 3 * n, *da = c->stage + 6 * n;
   if (c->precision == CVR_PREC_FP64)
@@ -2318,6 +2339,7 @@ int64_t cvr_get_sk(cvr_ctx *c, double *out) {
   if (!c->ewk_on) return 0;
   cudaSetDevice(c->device);
   if (out) {
+    if (int r = current_forces(c)) return -r;
     cudaError_t e = cudaMemcpyAsync(out, c->d_sk, (size_t)c->nk * sizeof(double2), cudaMemcpyDeviceToHost, c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) return -fail(c, CVR_ERR_CUDA, cudaGetErrorString(e));
