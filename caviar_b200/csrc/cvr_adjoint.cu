@@ -95,15 +95,15 @@ struct Params {
 };
 
 // Pair constants of the ordered type pair; the cutoffs^2 are in the units of
-// the tested displacements (mixed form: L / 2^32, which hh + hl turns into
-// lengths).
+// the tested displacements (fixed-point coordinates: L / 2^32).
 template <typename real> struct LjC {
   real sg2, e, shift, shiftS, U0, U1, S0, S1;
   int on;
 };
 template <typename real> struct PairC {
   real rl2, rr2;            // rr2 < 0: no Ewald
-  real hh, hl;
+  real rc2;                 // LJ cutoff^2 as a length
+  double unit;              // fixed-point unit
   real alpha, alpha2, beta, ke;
   LjC<real> lj[NTT];
 };
@@ -414,46 +414,81 @@ __global__ void __launch_bounds__(KRED_E *KRED_G) k_adj_kreduce(Params p, const 
 __device__ __forceinline__ float adj_rcp(float x) { return __fdividef(1.f, x); }
 __device__ __forceinline__ double adj_rcp(double x) { return 1.0 / x; }
 
-// The displacement r_j - r_i (minimum image) that the distance test uses and
-// the queues hold: mixed form, the wrapping difference of 32-bit fixed-point
-// coordinates in units L / 2^32 (pair_unit turns it into a length, correctly
-// rounded: one constant's rounding would shift every distance alike); FP64,
-// the difference itself.
-template <typename real> struct Coord;
-template <> struct Coord<float> {
+// Coordinates in the pair kernel: the displacement r_j - r_i (minimum image)
+// that the distance test takes (test) and the queues hold (Diff), and its
+// three lengths at the evaluation (length).
+//  FixedCoord  mixed form: the wrapping difference of 32-bit fixed-point
+//              coordinates in units L / 2^32, exact, turned into a length
+//              through FP64 with one rounding to FP32.
+//  WideCoord   mixed form in boxes where L / 2^32 is too coarse
+//              (FIXED_MAX_SIGMA): FP64 differences rounded once.
+//  FullCoord   FP64: the differences themselves.
+struct FixedCoord {
+  static constexpr int MIN_BLOCKS = 4;
+  struct Diff {
+    int x, y, z, j;
+  };
   uint32_t x, y, z;
   float bad;  // 0, or NaN where the position is not finite (a fixed-point coordinate cannot say so)
-  __device__ __forceinline__ static Coord load(const uint4 *xs, const double *, int, int j) {
+  __device__ __forceinline__ static FixedCoord load(const uint4 *xs, const double *, int, int j) {
     const uint4 v = xs[j];
     return {v.x, v.y, v.z, __uint_as_float(v.w)};
   }
-  __device__ __forceinline__ float3 to(const Coord &o, const Params &) const {
-    return make_float3((float)(int)(o.x - x) + o.bad, (float)(int)(o.y - y), (float)(int)(o.z - z));
+  __device__ __forceinline__ Diff to(const FixedCoord &o, const Params &, int j) const {
+    return {(int)(o.x - x), (int)(o.y - y), (int)(o.z - z), j};
   }
-};
-template <> struct Coord<double> {
-  double x, y, z;
-  static constexpr double bad = 0.0;  // the differences carry a NaN themselves
-  __device__ __forceinline__ static Coord load(const uint4 *, const double *X, int n, int j) {
-    return {X[j], X[n + j], X[2 * n + j]};
+  __device__ __forceinline__ static float test(const Diff &d, const FixedCoord &o) {
+    const float a = (float)d.x + o.bad, b = (float)d.y, c = (float)d.z;
+    return a * a + b * b + c * c;
   }
-  __device__ __forceinline__ double3 to(const Coord &o, const Params &p) const {
-    double3 d = make_double3(o.x - x, o.y - y, o.z - z);
-    d.x -= p.L * rint(d.x * p.invL);
-    d.y -= p.L * rint(d.y * p.invL);
-    d.z -= p.L * rint(d.z * p.invL);
+  // j's sign bit: the pair's r^2 was NaN
+  __device__ __forceinline__ static Diff marked(Diff d, float r2) {
+    if (r2 != r2) d.j |= 1 << 31;
     return d;
   }
+  template <typename PC> __device__ __forceinline__ static int length(const Diff &e, const PC &pc, float (&d)[3]) {
+    d[0] = (float)((double)e.x * pc.unit);
+    d[1] = (float)((double)e.y * pc.unit);
+    d[2] = (float)((double)e.z * pc.unit);
+    if (e.j < 0) d[0] = __int_as_float(0x7fffffff);
+    return e.j & 0x7fffffff;
+  }
 };
-template <typename real> struct Pair {  // a queued pair
+template <typename real> struct RealDiff {
   real x, y, z;
   int j;
 };
-__device__ __forceinline__ float pair_unit(float v, float hh, float hl) {
-  const float t = v * hh;
-  return t + fmaf(v, hl, fmaf(v, hh, -t));  // the product's rounding error and the unit's low part
-}
-__device__ __forceinline__ double pair_unit(double v, double, double) { return v; }
+template <typename real> struct RealCoord {
+  static constexpr int MIN_BLOCKS = sizeof(real) == 4 ? 3 : 2;  // 4 in the mixed form spill
+  using Diff = RealDiff<real>;
+  double x, y, z;
+  static constexpr double bad = 0.0;  // the differences carry a NaN themselves
+  __device__ __forceinline__ static RealCoord load(const uint4 *, const double *X, int n, int j) {
+    return {X[j], X[n + j], X[2 * n + j]};
+  }
+  __device__ __forceinline__ Diff to(const RealCoord &o, const Params &p, int j) const {
+    double d[3] = {o.x - x, o.y - y, o.z - z};
+#pragma unroll
+    for (int a = 0; a < 3; ++a) d[a] -= p.L * rint(d[a] * p.invL);
+    return {(real)d[0], (real)d[1], (real)d[2], j};
+  }
+  __device__ __forceinline__ static real test(const Diff &d, const RealCoord &) {
+    return d.x * d.x + d.y * d.y + d.z * d.z;
+  }
+  __device__ __forceinline__ static Diff marked(const Diff &d, real) { return d; }
+  template <typename PC> __device__ __forceinline__ static int length(const Diff &e, const PC &, real (&d)[3]) {
+    d[0] = e.x;
+    d[1] = e.y;
+    d[2] = e.z;
+    return e.j;
+  }
+};
+using WideCoord = RealCoord<float>;
+using FullCoord = RealCoord<double>;
+// Fixed-point coordinates in boxes of at most this many of the smallest LJ
+// diameter: FP32 rounds a contact distance to 1.7e-8 of it (r.m.s.), the two
+// coordinates' quanta add 9.5e-11 L / sigma, 1.6 % of that error at 32.
+constexpr double FIXED_MAX_SIGMA = 32.0;
 
 __device__ __forceinline__ void load_u(const float4 *us, const double *, int, int j, float (&u)[3]) {
   const float4 v = us[j];
@@ -499,13 +534,14 @@ __device__ __forceinline__ real apply(real c, real c1, const real (&d)[3], const
 // pipe).  4000 atoms, rc 8, mixed, with every lane evaluating its own partner
 // under divergence and FP64 differences: 216 us energy form with k space, 270
 // VJP; now 52 and 64 (+ 10 and 14 for the k-space kernel).
-template <typename real, bool VJP>
-__global__ void __launch_bounds__(PAIR_WARPS * 32, sizeof(real) == 4 ? 4 : 2)
+template <typename real, typename Coord, bool VJP>
+__global__ void __launch_bounds__(PAIR_WARPS * 32, Coord::MIN_BLOCKS)
     k_adj_pair(Params p, PairC<real> pc, const double *__restrict__ X, const double *__restrict__ U,
                const uint4 *__restrict__ xs, const float4 *__restrict__ us, int JS, double scale, double *__restrict__ out,
                double *__restrict__ part) {
   constexpr int PR = PAIR_ROUND<real>;
-  __shared__ Pair<real> queue[PAIR_WARPS][2][QCAP<real>];
+  using Diff = typename Coord::Diff;
+  __shared__ Diff queue[PAIR_WARPS][2][QCAP<real>];
   __shared__ double red[PAIR_WARPS][2][3];  // per warp, partner type
   __shared__ real facc[PAIR_WARPS][3];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -515,11 +551,11 @@ __global__ void __launch_bounds__(PAIR_WARPS * 32, sizeof(real) == 4 ? 4 : 2)
   const int ti = i >= p.n0;
   const bool param = scale != 0.0;
   const unsigned lt = (1u << lane) - 1u;
-  Pair<real> *qe = queue[warp][0], *ql = queue[warp][1];
+  Diff *qe = queue[warp][0], *ql = queue[warp][1];
   real acc[3] = {0, 0, 0}, ui[3] = {0, 0, 0};
   double sum[2][3] = {{0, 0, 0}, {0, 0, 0}};
   if (live) {
-    const Coord<real> ci = Coord<real>::load(xs, X, p.n, i);
+    const Coord ci = Coord::load(xs, X, p.n, i);
     if (VJP) load_u(us, U, p.n, i, ui);
     acc[0] = ci.bad;
 #pragma unroll
@@ -528,8 +564,8 @@ __global__ void __launch_bounds__(PAIR_WARPS * 32, sizeof(real) == 4 ? 4 : 2)
       const real qq = (real)((ti ? p.charge[1] : p.charge[0]) * p.charge[tj]);
       const int j0 = tj ? p.n0 : 0, j1 = tj ? p.n : p.n0;
       const auto ewald = [&](int k) {
-        const Pair<real> e = qe[k];
-        const real d[3] = {pair_unit(e.x, pc.hh, pc.hl), pair_unit(e.y, pc.hh, pc.hl), pair_unit(e.z, pc.hh, pc.hl)};
+        real d[3];
+        const int j = Coord::length(qe[k], pc, d);
         const real r2 = d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
         real r, ri, G, ec;
         if constexpr (sizeof(real) == 4) {
@@ -549,47 +585,47 @@ __global__ void __launch_bounds__(PAIR_WARPS * 32, sizeof(real) == 4 ? 4 : 2)
           const real E2 = pc.beta * G * ((real)2 * pc.alpha2 + (real)2 * ri * ri) + (real)2 * ec * ri * ri * ri;
           c1 = qq * pc.ke * (E2 - E1 * ri) * ri * ri;
         }
-        const real ud = apply<real, VJP>(qq * cq, c1, d, ui, us, U, p.n, e.j, acc);
+        const real ud = apply<real, VJP>(qq * cq, c1, d, ui, us, U, p.n, j, acc);
         if (param) sum[tj][2] += (double)(VJP ? cq * ud : pc.ke * ec * ri);
       };
       const auto lennard_jones = [&](int k) {
-        const Pair<real> e = ql[k];
-        const real d[3] = {pair_unit(e.x, pc.hh, pc.hl), pair_unit(e.y, pc.hh, pc.hl), pair_unit(e.z, pc.hh, pc.hl)};
+        real d[3];
+        const int j = Coord::length(ql[k], pc, d);
         const real r2 = d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
         const real r2i = adj_rcp(r2), s2 = lj.sg2 * r2i, s6 = s2 * s2 * s2, s12 = s6 * s6;
         const real ce = (real)4 * (((real)6 * s6 - (real)12 * s12) * r2i + lj.shift);
         const real c1 = VJP ? lj.e * (real)4 * ((real)168 * s12 - (real)48 * s6) * r2i * r2i : (real)0;
-        const real ud = apply<real, VJP>(lj.e * ce, c1, d, ui, us, U, p.n, e.j, acc);
+        const real ud = apply<real, VJP>(lj.e * ce, c1, d, ui, us, U, p.n, j, acc);
         if (param) {
           if (VJP) {
             const real cs = (real)4 * (((real)36 * s6 - (real)144 * s12) * r2i + lj.shiftS);
             sum[tj][0] += (double)(ce * ud);
             sum[tj][1] += (double)(cs * ud);
           } else {
-            sum[tj][0] += (double)((real)4 * (s12 - s6) + (lj.U0 + lj.U1 * r2));
-            sum[tj][1] += (double)((real)4 * ((real)12 * s12 - (real)6 * s6) + (lj.S0 + lj.S1 * r2));
+            sum[tj][0] += (double)((real)4 * (s12 - s6) + (lj.U0 + lj.U1 * (r2 - pc.rc2)));
+            sum[tj][1] += (double)((real)4 * ((real)12 * s12 - (real)6 * s6) + (lj.S0 + lj.S1 * (r2 - pc.rc2)));
           }
         }
       };
       int ne = 0, nl = 0;
       for (int b = j0 + 32 * PR * js; b < j1; b += 32 * PR * JS) {
-        Coord<real> cj[PR];
+        Coord cj[PR];
 #pragma unroll
-        for (int q = 0; q < PR; ++q) cj[q] = Coord<real>::load(xs, X, p.n, min(b + 32 * q + lane, p.n - 1));
+        for (int q = 0; q < PR; ++q) cj[q] = Coord::load(xs, X, p.n, min(b + 32 * q + lane, p.n - 1));
 #pragma unroll
         for (int q = 0; q < PR; ++q) {
           const int j = b + 32 * q + lane;
           const bool ok = j < j1 && j != i;
-          const auto d = ci.to(cj[q], p);
-          const real r2 = d.x * d.x + d.y * d.y + d.z * d.z;
+          const Diff d = ci.to(cj[q], p, j);
+          const real r2 = Coord::test(d, cj[q]);
           // a NaN (a position that is not finite) counts as inside, and so reaches the force
           const bool ie = ok && !(r2 > pc.rr2), il = ok && lj.on && r2 <= pc.rl2;
           const unsigned me = __ballot_sync(0xffffffffu, ie);
-          if (ie) qe[ne + __popc(me & lt)] = Pair<real>{d.x, d.y, d.z, j};
+          if (ie) qe[ne + __popc(me & lt)] = Coord::marked(d, r2);
           ne += __popc(me);
           const unsigned ml = __ballot_sync(0xffffffffu, il);
           if (ml) {
-            if (il) ql[nl + __popc(ml & lt)] = Pair<real>{d.x, d.y, d.z, j};
+            if (il) ql[nl + __popc(ml & lt)] = d;
             nl += __popc(ml);
           }
         }
@@ -824,6 +860,7 @@ struct cvr_adj {
   size_t ck_cap = 0, seg_cap = 0;
   int nch0 = 0, nch = 0, chunk = SK_STAGE;  // S(k) chunks: of type 0, of both; atoms per chunk
   int jsplit = 1;                           // warps per atom of k_adj_pair
+  bool fixed = false;                       // mixed form: fixed-point pair displacements
   PairC<float> pcf{};
   PairC<double> pcd{};
   std::string err;
@@ -897,8 +934,16 @@ int eval(cvr_adj *a, const PairC<real> &pc, const PrepArgs &prep, const double *
         p, a->skpart, a->nch0, a->nch, a->kw, kc, scale, VJP ? parts.kv : parts.ke);
     cudaEventRecord(a->join, a->kstream);
   }
-  k_adj_pair<real, VJP><<<pair_blocks(a), PAIR_WARPS * 32, 0, st>>>(p, pc, X, a->u, a->xs, a->us, a->jsplit, scale,
-                                                                    a->fp, VJP ? parts.pv : parts.pe);
+  const auto pair = [&](auto kernel) {
+    kernel<<<pair_blocks(a), PAIR_WARPS * 32, 0, st>>>(p, pc, X, a->u, a->xs, a->us, a->jsplit, scale, a->fp,
+                                                       VJP ? parts.pv : parts.pe);
+  };
+  if constexpr (sizeof(real) == 8)
+    pair(k_adj_pair<real, FullCoord, VJP>);
+  else if (a->fixed)
+    pair(k_adj_pair<real, FixedCoord, VJP>);
+  else
+    pair(k_adj_pair<real, WideCoord, VJP>);
   if (p.ncol > 0) cudaStreamWaitEvent(st, a->join, 0);
   k_adj_kforce<real, VJP><<<blocks(p.n, 32), KF_WARPS * 32, 0, st>>>(p, tab, kc, a->u, a->fp, post);
   return cuda_ok(a, "adjoint evaluation launch");
@@ -936,9 +981,8 @@ void sum_parts(cvr_adj *a, double *acc) {
 template <typename real>
 void set_pair_consts(const cvr_adj *a, double rc_lj, double rc_r, PairC<real> &c) {
   const Params &p = a->p;
-  const double unit = sizeof(real) == 4 ? p.L / 4294967296.0 : 1.0;
-  c.hh = (real)unit;
-  c.hl = (real)(unit - (double)c.hh);
+  const double unit = sizeof(real) == 4 && a->fixed ? p.L / 4294967296.0 : 1.0;
+  c.unit = unit;
   c.rl2 = (real)(rc_lj * rc_lj / (unit * unit));
   c.rr2 = (real)(p.k_e != 0.0 ? rc_r * rc_r / (unit * unit) : -1.0);
   c.alpha = (real)p.alpha;
@@ -946,6 +990,7 @@ void set_pair_consts(const cvr_adj *a, double rc_lj, double rc_r, PairC<real> &c
   c.beta = (real)(2.0 * p.alpha * 0.56418958354775628695);
   c.ke = (real)p.k_e;
   const double rc2 = rc_lj * rc_lj;
+  c.rc2 = (real)rc2;
   for (int x = 0; x < NT; ++x)
     for (int y = 0; y < NT; ++y) {
       LjC<real> &l = c.lj[x * NT + y];
@@ -959,9 +1004,9 @@ void set_pair_consts(const cvr_adj *a, double rc_lj, double rc_r, PairC<real> &c
       l.shiftS = (real)((144 * c12 - 36 * c6) / rc2);
       const double u1 = 4 * (12 * c12 - 6 * c6) / (2 * rc2), s1 = 4 * (144 * c12 - 36 * c6) / (2 * rc2);
       l.U1 = (real)u1;
-      l.U0 = (real)(-4 * (c12 - c6) - u1 * rc2);
+      l.U0 = (real)(-4 * (c12 - c6));
       l.S1 = (real)s1;
-      l.S0 = (real)(-4 * (12 * c12 - 6 * c6) - s1 * rc2);
+      l.S0 = (real)(-4 * (12 * c12 - 6 * c6));
     }
 }
 
@@ -1148,6 +1193,7 @@ int cvr_adj_set_params(cvr_adj *a, const double *charge, const double *eps, cons
   p.alpha = alpha;
   p.k_e = k_e;
   p.dt = dt;
+  a->fixed = a->precision == CVR_PREC_MIXED && p.L <= FIXED_MAX_SIGMA * *std::min_element(sigma, sigma + nt * nt);
   set_pair_consts(a, rc_lj, rc_r, a->pcf);
   set_pair_consts(a, rc_lj, rc_r, a->pcd);
   const bool kchanged = !a->params_set || kmax != p.kmax;
