@@ -87,10 +87,12 @@ struct BatchDev {
   const int *kinfo;
   double *out;  // [replica][NTH]
   // LJ lists: of replica r, entry k of atom i at list[LCAP * off[r] + k * n + i];
-  // neighbours per atom; coordinates at the build, SoA [3][atoms]
+  // neighbours per atom; coordinates at the build, SoA [3][atoms]; per replica
+  // whether its list is in use (carried between launches, as the forces are)
   uint16_t *list;
   int *list_count;
   uint32_t *list_u;
+  int *list_on;
   long long n_total;
   int nk, nruns, kmax, n_types;
   float eps[TMAX * TMAX], sig[TMAX * TMAX], charge[TMAX];
@@ -559,9 +561,10 @@ __device__ __forceinline__ void to_smem(const BatchDev &p, const Smem &S, int i,
 }
 
 // One launch: nsteps velocity-Verlet steps of replica order[first + blockIdx.x].
-// compute_first = 0 takes the forces of the current positions from fx/fy/fz
-// (written by the previous launch), so runs split over several launches are
-// bit-identical to one run.  Energies and virial come from a separate
+// compute_first = 0 takes the forces of the current positions and the LJ list
+// from the previous launch, so runs split over several launches are
+// bit-identical to one run.  A list that overflows is not tried again before
+// the next compute_first.  Energies and virial come from a separate
 // evaluation at the final positions (the stepping forces never depend on
 // whether energies are wanted).  Each thread owns atoms tid, tid + TPB, ...
 // for the integrator and the k-space force; the pair tiles write forces of
@@ -619,7 +622,7 @@ __global__ void __launch_bounds__(TPB, 1) k_batch(BatchDev p, int first, int nst
     const double half = 0.4999 * p.rc_lj[r] * LSKIN * 4294967296.0 / L;
     rl2 = (int)ceil(rl * rl);
     moved2 = (float)(half * half);
-    listed = build_lj_list<TPB>(p, S, n, o, rl2);
+    listed = compute_first ? build_lj_list<TPB>(p, S, n, o, rl2) : p.list_on[r] != 0;
   }
   double ev[5] = {0, 0, 0, 0, 0};
   if (compute_first) {
@@ -649,7 +652,7 @@ __global__ void __launch_bounds__(TPB, 1) k_batch(BatchDev p, int first, int nst
         X[a][gi] = x;
       }
       to_smem(p, S, i, gi, L);
-      if (wants_list) {
+      if (listed) {
         const float4 u = S.xh[i];
         const float dx = (float)(int)(__float_as_uint(u.x) - p.list_u[gi]),
                     dy = (float)(int)(__float_as_uint(u.y) - p.list_u[p.n_total + gi]),
@@ -667,7 +670,8 @@ __global__ void __launch_bounds__(TPB, 1) k_batch(BatchDev p, int first, int nst
       p.vz[gi] += h * (double)S.fsz[i] * mi;
     }
   }
-  // forces of the final positions, carried to the next launch
+  // forces of the final positions and the list's state, carried to the next launch
+  if (wants_list && threadIdx.x == 0) p.list_on[r] = listed;
   for (int i = threadIdx.x; i < n; i += TPB) {
     p.fx[o + i] = S.fsx[i];
     p.fy[o + i] = S.fsy[i];
@@ -935,7 +939,8 @@ int cvr_batch_create(cvr_batch **out, int n_rep, const int64_t *n_atoms, const d
   cudaMemset(farr, 0, 3 * N * sizeof(float));
   cudaMemset(dtype, 0, N * sizeof(int));
   uint16_t *list;
-  if ((rc = balloc(b, &list, (size_t)LCAP * N)) || (rc = balloc(b, &d.list_count, N)) || (rc = balloc(b, &d.list_u, 3 * N)))
+  if ((rc = balloc(b, &list, (size_t)LCAP * N)) || (rc = balloc(b, &d.list_count, N)) || (rc = balloc(b, &d.list_u, 3 * N)) ||
+      (rc = balloc(b, &d.list_on, n_rep)))
     return rc;
   d.list = list;
   d.n_total = o;
