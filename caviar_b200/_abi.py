@@ -25,6 +25,7 @@ N_THERMO = len(TH_KEYS)
 KT_PAIR, KT_KSPACE, KT_INTEGRATE, KT_BUILD = 0, 1, 2, 3
 LIST_AUTO, LIST_THREAD, LIST_WARP = 0, 1, 2
 KFORCE_AUTO, KFORCE_CUDA_CORES = 0, 1
+INJECT_BARRIER_POLLS = 1
 
 # Every symbol declared in include/caviar_b200.h.
 EXPORTED = ["cvr_create", "cvr_destroy", "cvr_set_neighborlist", "cvr_set_lj", "cvr_set_ewald_r", "cvr_set_ewald_k",
@@ -38,7 +39,7 @@ EXPORTED = ["cvr_create", "cvr_destroy", "cvr_set_neighborlist", "cvr_set_lj", "
             "cvr_batch_last_error", "cvr_batch_stream", "cvr_adj_create", "cvr_adj_destroy", "cvr_adj_set_params",
             "cvr_adj_set_state", "cvr_adj_forces", "cvr_adj_force_vjp", "cvr_adj_loss", "cvr_adj_loss_grad",
             "cvr_adj_last_error", "cvr_adj_stream", "cvr_measure_fma_peak", "cvr_set_lj_jump_tol",
-            "cvr_set_all_atom_test"]
+            "cvr_set_all_atom_test", "cvr_inject_failure"]
 
 _dp = ctypes.POINTER(ctypes.c_double)
 _ip = ctypes.POINTER(ctypes.c_int32)
@@ -323,6 +324,11 @@ class Simulation:
     def set_kspace_force_kernel(self, kind: int):
         """KFORCE_AUTO (tensor cores where they apply) or KFORCE_CUDA_CORES."""
         self._check(self.L.cvr_set_kspace_force_kernel(self.h, kind))
+
+    def inject_failure(self, kind: int, value: int):
+        """INJECT_BARRIER_POLLS: most polls of a wait between a launch's blocks (0: the default)."""
+        self.L.cvr_inject_failure.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_int64]
+        self._check(self.L.cvr_inject_failure(self.h, kind, value))
 
     def set_kernel_timing(self, on: bool):
         self._check(self.L.cvr_set_kernel_timing(self.h, int(on)))

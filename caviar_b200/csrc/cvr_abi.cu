@@ -199,6 +199,7 @@ struct cvr_ctx {
   unsigned long long *step_ctrl{};
   double *step_part{}, *step_rec{}, *step_pos{};
   int step_launch = 0;
+  unsigned barrier_polls = BARRIER_POLLS;
   int64_t steps_n = 0;  // atoms the buffers are sized for
   // Langevin integrator (md_simulator.cpp:670-811)
   int integrator = 0;  // 0 velocity Verlet, 1 velocity Verlet Langevin
@@ -1017,7 +1018,7 @@ int launch_build_now(cvr_ctx *c, int count_only) {
   CVR_CUDA(c, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int log2_tpa = c->log2_tpa, launch = c->step_launch;
   c->step_launch ^= 1;
-  void *args[] = {&s, &c->step_ctrl, &launch, &count_only, &log2_tpa};
+  void *args[] = {&s, &c->step_ctrl, &launch, &c->barrier_polls, &count_only, &log2_tpa};
   CVR_CUDA(c, cudaLaunchCooperativeKernel((const void *)kernel, dim3(g.grid), dim3(g.threads), args, smem, c->stream));
   c->launches++;
   if (phase_in_drift(c)) {  // the atoms moved in memory: the step's phase tables follow them
@@ -1054,8 +1055,15 @@ int read_flags(cvr_ctx *c, int out[4]) {
   CVR_CUDA(c, cudaStreamSynchronize(c->stream));
   if (out != c->back->flags) std::memcpy(out, c->back->flags, 4 * sizeof(int));
   c->builds_seen = c->back->flags[3];
-  if (c->back->flags[1] & ERR_BARRIER) {  // the barrier words start again from zero
+  if (c->back->flags[1] & ERR_BARRIER) {
+    // the blocks left in the middle of a step or a build: the flags, the
+    // barrier words and the build's counters start again from zero, the state is gone
+    cudaMemsetAsync(c->flags, 0, 4 * sizeof(int), c->stream);
+    c->builds_seen = 0;
     cudaMemsetAsync(c->step_ctrl, 0, SC_WORDS * sizeof(unsigned long long), c->stream);
+    cudaMemsetAsync(c->cell_count, 0, ((size_t)c->ncells + 1) * sizeof(int), c->stream);
+    cudaMemsetAsync(c->cell_fill, 0, ((size_t)c->ncells + 1) * sizeof(int), c->stream);
+    c->have_state = c->list_valid = c->setup_done = c->list_fresh = false;
     return fail(c, CVR_ERR_CUDA, "a grid barrier's wait ran out");
   }
   return CVR_OK;
@@ -1362,6 +1370,7 @@ int launch_steps_t(cvr_ctx *c, int nsteps, int64_t every, int64_t done) {
   a.bz = a.by + c->n;
   a.ctrl = c->step_ctrl;
   a.launch = c->step_launch;
+  a.polls = c->barrier_polls;
   c->step_launch ^= 1;
   a.counters = c->counters;
   a.ts = thermostat_args(c);
@@ -2119,11 +2128,23 @@ int cvr_set_list_kernel(cvr_ctx *c, int kind) {
   return CVR_OK;
 }
 
+int cvr_inject_failure(cvr_ctx *c, int kind, int64_t value) {
+  if (!c) return CVR_ERR_INVALID;
+  if (kind != CVR_INJECT_BARRIER_POLLS || value < 0 || value > BARRIER_POLLS)
+    return fail(c, CVR_ERR_INVALID, "unknown failure or value out of range");
+  c->barrier_polls = value ? (unsigned)value : BARRIER_POLLS;
+  return CVR_OK;
+}
+
 int cvr_set_precision(cvr_ctx *c, int precision) {
   if (!c) return CVR_ERR_INVALID;
   if (precision != CVR_PREC_MIXED && precision != CVR_PREC_FP64) return fail(c, CVR_ERR_INVALID, "unknown precision");
   if (c->have_state && precision != c->precision)
     return fail(c, CVR_ERR_STATE, "precision must be chosen before cvr_set_state");
+  if (precision != c->precision) {  // what a failed cvr_set_state or run left behind is the other precision's
+    c->n = 0;
+    c->refreshed = false;
+  }
   c->precision = precision;
   return CVR_OK;
 }

@@ -26,7 +26,9 @@
 // summed in another order).
 //
 // The barriers' waits are bounded; one that runs out sets ERR_BARRIER and the
-// block leaves.
+// block leaves.  A block passes a barrier only when all have arrived at it, so
+// the blocks still running never see a stage half done; the state and the
+// build's counters are left as they are, and the host drops both.
 #pragma once
 #include "cvr_build.cuh"
 #include "cvr_device.cuh"
@@ -54,6 +56,7 @@ template <typename real> struct StepArgs {
   double *bx, *by, *bz;       // positions at the build
   unsigned long long *ctrl;
   int launch;                 // parity: which pair of control words is this launch's
+  unsigned polls;             // most polls of a barrier's wait
   long long *counters;
   ThermostatArgs ts;
   double *part;               // [gridDim.x][4]: the thermostat's block sums
@@ -64,7 +67,7 @@ template <typename real> struct StepArgs {
   ThermoArgs th;
 };
 
-constexpr unsigned BARRIER_POLLS = 1u << 22;  // some seconds
+constexpr unsigned BARRIER_POLLS = 1u << 22;  // a barrier's wait: some seconds
 constexpr int STEPS_MAX = 1 << 16;            // steps per launch (the need field's range)
 
 // Grid barrier on a counter per parity of the barrier: every block adds 1,
@@ -78,13 +81,15 @@ struct GridBarrier {
   unsigned long long *word;  // [2]
   unsigned count[2];         // arrivals awaited, per parity
   unsigned needs[2];         // rebuild requests before this barrier, per parity
+  unsigned limit;            // most polls of a wait
   int parity;
   int need, bad;             // set by any thread that asks for a rebuild or met an error
   int answer;
 
-  __device__ __forceinline__ void init(unsigned long long *w) {
+  __device__ __forceinline__ void init(unsigned long long *w, unsigned polls) {
     if (threadIdx.x == 0) {
       word = w;
+      limit = polls;
       count[0] = count[1] = needs[0] = needs[1] = 0;
       parity = need = bad = 0;
     }
@@ -106,7 +111,7 @@ struct GridBarrier {
       unsigned polls = 0;
       do {
         asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(w) : "memory");
-      } while ((unsigned)v < want && ++polls < BARRIER_POLLS);
+      } while ((unsigned)v < want && ++polls < limit);
       int a = (v >> 56) ? 2 : 0;
       if ((unsigned)v < want) {
         atomicOr(err, ERR_BARRIER);
@@ -202,7 +207,7 @@ __global__ void __launch_bounds__(STEP_THREADS, 1) k_steps(DevState<real> s, Ste
   const int gwarp = blockIdx.x * WARPS + warp, nwarps = gridDim.x * WARPS;
   for (int t = threadIdx.x; t < (ONE_TYPE ? 1 : s.n_types * s.n_types); t += THREADS) coef[t] = a.coef[t];
   if (tid < 2) a.ctrl[2 * (a.launch ^ 1) + tid] = 0;
-  grid.init(a.ctrl + 2 * a.launch);
+  grid.init(a.ctrl + 2 * a.launch, a.polls);
   const Stencil<real> st = stencil_of(s);
   const EwrArgs<real> no_ewald{};
   const WarpPieces wp = warp_pieces(smraw, warp, WARPS);
@@ -470,7 +475,7 @@ __global__ void __launch_bounds__(STEP_THREADS, 1) k_steps(DevState<real> s, Ste
 // at once if the rebuild flag is not set.
 template <typename real>
 __global__ void __launch_bounds__(STEP_THREADS, 1)
-    k_build_once(DevState<real> s, unsigned long long *ctrl, int launch, int count_only, int log2_tpa) {
+    k_build_once(DevState<real> s, unsigned long long *ctrl, int launch, unsigned polls, int count_only, int log2_tpa) {
   extern __shared__ __align__(16) unsigned char smraw[];
   __shared__ GridBarrier grid;
   __shared__ int red[STEP_THREADS / 32];
@@ -478,7 +483,7 @@ __global__ void __launch_bounds__(STEP_THREADS, 1)
   const int tid = blockIdx.x * blockDim.x + threadIdx.x, nthreads = gridDim.x * blockDim.x;
   if (tid < 2) ctrl[2 * (launch ^ 1) + tid] = 0;
   if (*s.flag == 0) return;
-  grid.init(ctrl + 2 * launch);
+  grid.init(ctrl + 2 * launch, polls);
   for (int i = tid; i < n; i += nthreads) bin_atom(s, i);
   if (grid.meet(s.err) & 2) return;
   if (tid == 0) {

@@ -172,6 +172,14 @@ int cvr_set_kspace_force_kernel(cvr_ctx *ctx, int kind);
 #define CVR_LIST_WARP 2
 int cvr_set_list_kernel(cvr_ctx *ctx, int kind);
 
+/* Failures on the host's request, for tests of what follows them (no
+ * reference counterpart).  CVR_INJECT_BARRIER_POLLS: the most polls of a wait
+ * between the blocks of a launch that runs many steps or a list build (0: the
+ * default, some seconds); a wait that runs out fails the call with
+ * CVR_ERR_CUDA and the state has to be set again. */
+#define CVR_INJECT_BARRIER_POLLS 1
+int cvr_inject_failure(cvr_ctx *ctx, int kind, int64_t value);
+
 /* CVR_PREC_MIXED (default) or CVR_PREC_FP64.  No reference counterpart
  * (the reference is FP64 only).  In the mixed form, a cubic box whose listed
  * pairs stay below L/2 apart and that has at most 256 cells per axis gets
