@@ -25,7 +25,7 @@ N_THERMO = len(TH_KEYS)
 KT_PAIR, KT_KSPACE, KT_INTEGRATE, KT_BUILD = 0, 1, 2, 3
 LIST_AUTO, LIST_THREAD, LIST_WARP = 0, 1, 2
 KFORCE_AUTO, KFORCE_CUDA_CORES = 0, 1
-INJECT_BARRIER_POLLS = 1
+INJECT_BARRIER_POLLS, INJECT_LAUNCH_ERROR = 1, 2
 
 # Every symbol declared in include/caviar_b200.h.
 EXPORTED = ["cvr_create", "cvr_destroy", "cvr_set_neighborlist", "cvr_set_lj", "cvr_set_ewald_r", "cvr_set_ewald_k",
@@ -326,7 +326,8 @@ class Simulation:
         self._check(self.L.cvr_set_kspace_force_kernel(self.h, kind))
 
     def inject_failure(self, kind: int, value: int):
-        """INJECT_BARRIER_POLLS: most polls of a wait between a launch's blocks (0: the default)."""
+        """INJECT_BARRIER_POLLS: most polls of a wait between a launch's blocks (0: the default);
+        INJECT_LAUNCH_ERROR: what the next such launch gives instead of being made."""
         self.L.cvr_inject_failure.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_int64]
         self._check(self.L.cvr_inject_failure(self.h, kind, value))
 

@@ -200,6 +200,8 @@ struct cvr_ctx {
   double *step_part{}, *step_rec{}, *step_pos{};
   int step_launch = 0;
   unsigned barrier_polls = BARRIER_POLLS;
+  bool cooperative = true;                 // false once the driver refused a cooperative launch
+  cudaError_t inject_launch = cudaSuccess;  // what the next one returns instead (cvr_inject_failure)
   int64_t steps_n = 0;  // atoms the buffers are sized for
   // Langevin integrator (md_simulator.cpp:670-811)
   int integrator = 0;  // 0 velocity Verlet, 1 velocity Verlet Langevin
@@ -1003,24 +1005,45 @@ GridShape grid_shape(const cvr_ctx *c, int groups) {
   return g;
 }
 
+// Launches a kernel that meets at grid barriers.  The parity of its barrier
+// words moves on only when it was launched: it clears the next launch's pair.
+// LAUNCH_REFUSED where the driver will not hold the whole grid resident (part
+// of the GPU is taken from the process): the caller takes one kernel per stage,
+// as every later call does.
+constexpr int LAUNCH_REFUSED = -1;
+int launch_cooperative(cvr_ctx *c, const void *kernel, const GridShape &g, void **args, size_t smem) {
+  CVR_CUDA(c, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  cudaError_t e = c->inject_launch;
+  c->inject_launch = cudaSuccess;
+  if (e == cudaSuccess)
+    e = cudaLaunchCooperativeKernel(kernel, dim3(g.grid), dim3(g.threads), args, smem, c->stream);
+  if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported) {
+    cudaGetLastError();
+    c->cooperative = false;
+    return LAUNCH_REFUSED;
+  }
+  CVR_CUDA(c, e);
+  c->step_launch ^= 1;
+  c->launches++;
+  return CVR_OK;
+}
+
 // A list build outside the step loop: one launch (k_build_once) for the
 // systems whose lists a warp per atom searches, else launch_build's.
 template <typename real>
 int launch_build_now(cvr_ctx *c, int count_only) {
-  if (c->timing || c->n > STEPS_MAX_ATOMS || list_kernel_kind(c) != CVR_LIST_WARP) {
+  if (c->timing || !c->cooperative || c->n > STEPS_MAX_ATOMS || list_kernel_kind(c) != CVR_LIST_WARP) {
     launch_build<real>(c, count_only);
     return CVR_OK;
   }
   DevState<real> s = dev_state<real>(c);
   const GridShape g = grid_shape(c, (int)c->n);
   const size_t smem = steps_smem(g.threads / 32);
-  auto kernel = k_build_once<real>;
-  CVR_CUDA(c, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int log2_tpa = c->log2_tpa, launch = c->step_launch;
-  c->step_launch ^= 1;
   void *args[] = {&s, &c->step_ctrl, &launch, &c->barrier_polls, &count_only, &log2_tpa};
-  CVR_CUDA(c, cudaLaunchCooperativeKernel((const void *)kernel, dim3(g.grid), dim3(g.threads), args, smem, c->stream));
-  c->launches++;
+  const int r = launch_cooperative(c, (const void *)k_build_once<real>, g, args, smem);
+  if (r == LAUNCH_REFUSED) launch_build<real>(c, count_only);
+  if (r != CVR_OK) return r == LAUNCH_REFUSED ? CVR_OK : r;
   if (phase_in_drift(c)) {  // the atoms moved in memory: the step's phase tables follow them
     k_phase<real><<<grid_for(3 * (int64_t)c->n, 256), 256, 0, c->stream>>>(s, kargs<real>(c), s.flag);
     c->launches++;
@@ -1341,7 +1364,8 @@ int stage_reference_eta(cvr_ctx *c, int slot) {
 // chain, the Langevin noise and the debug modes keep one kernel per stage)
 // and a system whose list is searched by a warp per atom.
 bool steps_in_one(const cvr_ctx *c) {
-  return c->use_graphs && !c->timing && c->lj_on && !c->ewr_on && !(c->ewk_on && c->nk > 0) && !c->all_atom &&
+  return c->use_graphs && !c->timing && c->cooperative && c->lj_on && !c->ewr_on && !(c->ewk_on && c->nk > 0) &&
+         !c->all_atom &&
          c->integrator == 0 && !c->sc_on && !(c->ewk_on && c->dipole_mode) && c->n <= STEPS_MAX_ATOMS &&
          (c->tpa == 32 || c->tpa == 8) && list_kernel_kind(c) == CVR_LIST_WARP;
 }
@@ -1371,7 +1395,6 @@ int launch_steps_t(cvr_ctx *c, int nsteps, int64_t every, int64_t done) {
   a.ctrl = c->step_ctrl;
   a.launch = c->step_launch;
   a.polls = c->barrier_polls;
-  c->step_launch ^= 1;
   a.counters = c->counters;
   a.ts = thermostat_args(c);
   a.part = c->step_part;
@@ -1384,12 +1407,8 @@ int launch_steps_t(cvr_ctx *c, int nsteps, int64_t every, int64_t done) {
   if (every > 0) a.th = thermo_args(c, c->d_thermo);
   DevState<real> s = dev_state<real>(c);
   const size_t smem = steps_smem(g.threads / 32);
-  auto kernel = k_steps<real, TPA, ONE_TYPE, FIXED>;
-  CVR_CUDA(c, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   void *args[] = {&s, &a};
-  CVR_CUDA(c, cudaLaunchCooperativeKernel((const void *)kernel, dim3(g.grid), dim3(g.threads), args, smem, c->stream));
-  c->launches++;
-  return CVR_OK;
+  return launch_cooperative(c, (const void *)k_steps<real, TPA, ONE_TYPE, FIXED>, g, args, smem);
 }
 
 template <typename real, bool FIXED>
@@ -1537,16 +1556,21 @@ int run_impl(cvr_ctx *c, int64_t nsteps, int64_t every, double *thermo) {
         c->ndist[a] = nd0[a];
       }
     }
-    const bool in_one = graphs && steps_in_one(c);
+    int64_t k0 = 0;  // steps done in launches of many
+    while (graphs && k0 < nsteps && steps_in_one(c)) {
+      const int chunk = (int)std::min<int64_t>(nsteps - k0, STEPS_MAX);
+      const int r = launch_steps<real>(c, chunk, every, k0);
+      if (r == CVR_OK) k0 += chunk;
+      else if (r != LAUNCH_REFUSED) return r;
+    }
+    const bool in_one = k0 == nsteps;
     const bool dk = defer_kick(c);
     if (graphs && !in_one && (c->graph_epoch != c->epoch || (dk && !c->g_step[1][0])))
       if (int r = build_graphs<real>(c)) return r;
     const int64_t launches0 = c->launches;
     bool pending = false;  // the previous step deferred its second half kick
     int64_t n_kick = 0;    // steps ending with a plain (no thermo) kick
-    for (int64_t k = 0; in_one && k < nsteps; k += STEPS_MAX)
-      if (int r = launch_steps<real>(c, (int)std::min<int64_t>(nsteps - k, STEPS_MAX), every, k)) return r;
-    for (int64_t k = in_one ? nsteps : 0; k < nsteps; ++k) {
+    for (int64_t k = k0; k < nsteps; ++k) {
       const bool th = every > 0 && ((k + 1) % every == 0);
       const int tail = th ? 2 : ((dk && k + 1 < nsteps) ? 0 : 1);
       n_kick += tail == 1;
@@ -1576,7 +1600,7 @@ int run_impl(cvr_ctx *c, int64_t nsteps, int64_t every, double *thermo) {
       const int tail = (c->lj_on || c->ewr_on ? 1 : 0) + ks + ((c->tstat.kind && c->integrator == 0) ? 2 : 0) +
                        (c->sc_on ? 4 : 0) + ((c->ewk_on && c->dipole_mode) ? 3 : 0);
       const int kick_plain = kick_in_kforce(c, false) ? 0 : 1;
-      c->launches = launches0 + nsteps * (2 + tail) + n_kick * kick_plain + nrec * 2 +
+      c->launches = launches0 + (nsteps - k0) * (2 + tail) + n_kick * kick_plain + nrec * 2 +
                     (8 + (phase_in_drift(c) ? 1 : 0)) * (int64_t)(f[3] - builds0);
     }
     if (f[1] & ERR_NAN) return fail(c, CVR_ERR_NAN, "NaN acceleration");
@@ -2130,10 +2154,15 @@ int cvr_set_list_kernel(cvr_ctx *c, int kind) {
 
 int cvr_inject_failure(cvr_ctx *c, int kind, int64_t value) {
   if (!c) return CVR_ERR_INVALID;
-  if (kind != CVR_INJECT_BARRIER_POLLS || value < 0 || value > BARRIER_POLLS)
-    return fail(c, CVR_ERR_INVALID, "unknown failure or value out of range");
-  c->barrier_polls = value ? (unsigned)value : BARRIER_POLLS;
-  return CVR_OK;
+  if (kind == CVR_INJECT_BARRIER_POLLS && value >= 0 && value <= BARRIER_POLLS) {
+    c->barrier_polls = value ? (unsigned)value : BARRIER_POLLS;
+    return CVR_OK;
+  }
+  if (kind == CVR_INJECT_LAUNCH_ERROR && value >= 0 && value <= 999) {
+    c->inject_launch = (cudaError_t)value;
+    return CVR_OK;
+  }
+  return fail(c, CVR_ERR_INVALID, "unknown failure or value out of range");
 }
 
 int cvr_set_precision(cvr_ctx *c, int precision) {

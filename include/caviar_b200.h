@@ -176,8 +176,12 @@ int cvr_set_list_kernel(cvr_ctx *ctx, int kind);
  * reference counterpart).  CVR_INJECT_BARRIER_POLLS: the most polls of a wait
  * between the blocks of a launch that runs many steps or a list build (0: the
  * default, some seconds); a wait that runs out fails the call with
- * CVR_ERR_CUDA and the state has to be set again. */
+ * CVR_ERR_CUDA and the state has to be set again.  CVR_INJECT_LAUNCH_ERROR:
+ * the CUDA error code that the next such launch gives instead of being made.
+ * 720 and 801 are a refusal: the context takes one kernel per stage from
+ * there on; any other code fails the call. */
 #define CVR_INJECT_BARRIER_POLLS 1
+#define CVR_INJECT_LAUNCH_ERROR 2
 int cvr_inject_failure(cvr_ctx *ctx, int kind, int64_t value);
 
 /* CVR_PREC_MIXED (default) or CVR_PREC_FP64.  No reference counterpart
