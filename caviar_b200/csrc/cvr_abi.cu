@@ -2197,6 +2197,17 @@ int cvr_set_state(cvr_ctx *c, int64_t n, const double *pos, const double *vel, c
   // every type, and the charge and mass sums at one term per type): the
   // staged arrays reach the state only if the check passes.  The velocities
   // follow on the side stream and reach the atoms' places by id at the end.
+  // The host arrays are borrowed for this call only: the copies from them
+  // (asynchronous when they are pinned) end before it returns, however it does.
+  struct Borrowed {
+    cvr_ctx *c;
+    bool over = false;
+    ~Borrowed() {
+      if (over) return;
+      cudaStreamSynchronize(c->kstream);
+      cudaStreamSynchronize(c->stream);
+    }
+  } borrowed{c};
   CVR_CUDA(c, cudaMemcpyAsync(c->stage_i, type, (size_t)n * sizeof(int32_t), cudaMemcpyHostToDevice, c->stream));
   CVR_CUDA(c, cudaMemsetAsync(c->d_type_hist, 0, (MAX_TYPES + 1) * sizeof(unsigned long long), c->stream));
   k_type_hist<<<std::min<int64_t>(grid_for(n, 256), 4 * 148), 256, 0, c->stream>>>(c->stage_i, (int)n, c->n_types,
@@ -2228,12 +2239,12 @@ int cvr_set_state(cvr_ctx *c, int64_t n, const double *pos, const double *vel, c
   };
   if (!kept) {
     if (int r = read_types()) return r;
-    if (c->back->per_type[MAX_TYPES] != 0) {
-      cudaStreamSynchronize(c->kstream);  // the caller's velocity array is borrowed until the copy ends
-      return fail(c, CVR_ERR_INVALID, "atom type out of range");
-    }
+    if (c->back->per_type[MAX_TYPES] != 0) return fail(c, CVR_ERR_INVALID, "atom type out of range");
     c->use_mol = mol != nullptr;
   }
+  // from here until the sums below no state counts, should the call fail in between
+  const bool list_was_valid = c->list_valid;
+  c->have_state = c->list_valid = false;
   if (c->precision == CVR_PREC_FP64)
     k_scatter_state<double><<<grid_for(n, 256), 256, 0, c->stream>>>(dev_state<double>(c), c->stage, nullptr,
                                                                       c->stage_i, mol_d, kept ? bad : nullptr);
@@ -2269,8 +2280,6 @@ int cvr_set_state(cvr_ctx *c, int64_t n, const double *pos, const double *vel, c
     sums();
     rs = (!c->refreshed || mol_changed) ? refresh(c) : DISPATCH(c, setup_run, c);
   }
-  // the host arrays are borrowed for this call only: the copies from them
-  // (asynchronous when they are pinned) end before it returns
   cudaError_t e = cudaStreamWaitEvent(c->stream, c->k_join, 0);
   if (vel && e == cudaSuccess) {
     if (c->precision == CVR_PREC_FP64)
@@ -2284,7 +2293,11 @@ int cvr_set_state(cvr_ctx *c, int64_t n, const double *pos, const double *vel, c
   if (kept && e == cudaSuccess) {
     e = cudaMemsetAsync(c->flags, 0, sizeof(int), c->stream);  // the build is done
     if (int r = read_types()) return r;
-    if (c->back->per_type[MAX_TYPES] != 0) return fail(c, CVR_ERR_INVALID, "atom type out of range");
+    if (c->back->per_type[MAX_TYPES] != 0) {  // nothing was written
+      c->have_state = true;
+      c->list_valid = list_was_valid;
+      return fail(c, CVR_ERR_INVALID, "atom type out of range");
+    }
     sums();
     int f = c->back->flags[1];
     // a denser state than the list was sized for
@@ -2299,6 +2312,7 @@ int cvr_set_state(cvr_ctx *c, int64_t n, const double *pos, const double *vel, c
     c->list_valid = c->list_fresh = true;
   }
   const cudaError_t e2 = cudaStreamSynchronize(c->stream);
+  borrowed.over = e == cudaSuccess && e2 == cudaSuccess;
   if (e == cudaSuccess) e = e2;
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) return fail(c, CVR_ERR_CUDA, cudaGetErrorString(e));
