@@ -883,8 +883,20 @@ template <typename T>
 int dalloc(cvr_adj *a, T **ptr, size_t count) {
   if (*ptr) cudaFree(*ptr);
   *ptr = nullptr;
-  if (cudaMalloc((void **)ptr, std::max<size_t>(count, 1) * sizeof(T)) != cudaSuccess)
+  if (cudaMalloc((void **)ptr, std::max<size_t>(count, 1) * sizeof(T)) != cudaSuccess) {
+    cudaGetLastError();  // not the next launch's
+    *ptr = nullptr;
     return afail(a, CVR_ERR_NOMEM, "cudaMalloc");
+  }
+  return CVR_OK;
+}
+
+// At least count doubles in *ptr (an allocation that fails leaves none).
+int reserve(cvr_adj *a, double **ptr, size_t *cap, size_t count) {
+  if (count <= *cap) return CVR_OK;
+  *cap = 0;
+  if (int rc = dalloc(a, ptr, count)) return rc;
+  *cap = count;
   return CVR_OK;
 }
 
@@ -1197,6 +1209,7 @@ int cvr_adj_set_params(cvr_adj *a, const double *charge, const double *eps, cons
   set_pair_consts(a, rc_lj, rc_r, a->pcf);
   set_pair_consts(a, rc_lj, rc_r, a->pcd);
   const bool kchanged = !a->params_set || kmax != p.kmax;
+  a->params_set = false;  // until everything below is done
   p.kmax = kmax;
   p.kp = kmax + 1;
   p.M = kmax + 1;
@@ -1236,7 +1249,9 @@ int cvr_adj_set_params(cvr_adj *a, const double *charge, const double *eps, cons
     a->kc = q + tab_d;
     a->parts = q + tab_d + kc_d;
   }
-  if (!kw.empty()) cudaMemcpy(a->kw, kw.data(), kw.size() * sizeof(double2), cudaMemcpyHostToDevice);
+  if (!kw.empty() &&
+      cudaMemcpy(a->kw, kw.data(), kw.size() * sizeof(double2), cudaMemcpyHostToDevice) != cudaSuccess)
+    return afail(a, CVR_ERR_CUDA, "k-space weights");
   a->params_set = true;
   return CVR_OK;
 }
@@ -1371,14 +1386,8 @@ int cvr_adj_loss_grad(cvr_adj *a, int64_t nsteps, int64_t checkpoint_every, doub
   const size_t N3 = 3 * (size_t)a->p.n, B3 = N3 * sizeof(double);
   const int64_t M = nsteps, K = std::min<int64_t>(checkpoint_every, nsteps);
   const int64_t nseg = (M + K - 1) / K, last0 = (nseg - 1) * K;
-  if ((size_t)nseg * 3 * N3 > a->ck_cap) {
-    if (int rc = dalloc(a, &a->ck, (size_t)nseg * 3 * N3)) return rc;
-    a->ck_cap = (size_t)nseg * 3 * N3;
-  }
-  if ((size_t)(K + 1) * 2 * N3 > a->seg_cap) {
-    if (int rc = dalloc(a, &a->seg, (size_t)(K + 1) * 2 * N3)) return rc;
-    a->seg_cap = (size_t)(K + 1) * 2 * N3;
-  }
+  if (int rc = reserve(a, &a->ck, &a->ck_cap, (size_t)nseg * 3 * N3)) return rc;
+  if (int rc = reserve(a, &a->seg, &a->seg_cap, (size_t)(K + 1) * 2 * N3)) return rc;
   double *segX = a->seg, *segF = a->seg + (size_t)(K + 1) * N3;
   cudaStream_t st = a->stream;
   const double invM = 1.0 / (double)M;
