@@ -19,8 +19,8 @@
 //   Gr -= F(r')/M;  Ga += dt/2 Gv;  Gr += (dF/dr)^T (Ga/m);  theta_bar += (dF/dtheta)^T (Ga/m)
 //   (Gr, Gv, Ga) <- (Gr, Gv + dt Gr, dt/2 Gv + dt^2/2 Gr)
 // and finally the VJP at r_0 for a_0 = F(r_0)/m.  Positions, velocities and
-// forces are checkpointed every K steps; the reverse sweep re-runs each
-// segment forward, keeping its K positions and forces (the last segment's
+// (memory allowing) forces are checkpointed every K steps; the reverse sweep
+// re-runs each segment forward, keeping its K positions and forces (the last segment's
 // are kept by the forward pass itself).
 //
 // Atoms are stored sorted by type (type 0 first), so that the partners of
@@ -1386,7 +1386,13 @@ int cvr_adj_loss_grad(cvr_adj *a, int64_t nsteps, int64_t checkpoint_every, doub
   const size_t N3 = 3 * (size_t)a->p.n, B3 = N3 * sizeof(double);
   const int64_t M = nsteps, K = std::min<int64_t>(checkpoint_every, nsteps);
   const int64_t nseg = (M + K - 1) / K, last0 = (nseg - 1) * K;
-  if (int rc = reserve(a, &a->ck, &a->ck_cap, (size_t)nseg * 3 * N3)) return rc;
+  // a checkpoint holds positions and velocities, and the forces (which save an
+  // evaluation per segment) where memory allows
+  size_t ckn = 3;
+  if (reserve(a, &a->ck, &a->ck_cap, (size_t)nseg * 3 * N3) != CVR_OK) {
+    ckn = 2;
+    if (int rc = reserve(a, &a->ck, &a->ck_cap, (size_t)nseg * 2 * N3)) return rc;
+  }
   if (int rc = reserve(a, &a->seg, &a->seg_cap, (size_t)(K + 1) * 2 * N3)) return rc;
   double *segX = a->seg, *segF = a->seg + (size_t)(K + 1) * N3;
   cudaStream_t st = a->stream;
@@ -1400,10 +1406,10 @@ int cvr_adj_loss_grad(cvr_adj *a, int64_t nsteps, int64_t checkpoint_every, doub
   if (int rc = eval_forces(a, x, f, 0.0)) return rc;
   for (int64_t t = 0; t < M; ++t) {
     if (t % K == 0 && t < last0) {
-      double *c = a->ck + (size_t)(t / K) * 3 * N3;
+      double *c = a->ck + (size_t)(t / K) * ckn * N3;
       cudaMemcpyAsync(c, x, B3, cudaMemcpyDeviceToDevice, st);
-      cudaMemcpyAsync(c + N3, f, B3, cudaMemcpyDeviceToDevice, st);
-      cudaMemcpyAsync(c + 2 * N3, a->V, B3, cudaMemcpyDeviceToDevice, st);
+      cudaMemcpyAsync(c + N3, a->V, B3, cudaMemcpyDeviceToDevice, st);
+      if (ckn == 3) cudaMemcpyAsync(c + 2 * N3, f, B3, cudaMemcpyDeviceToDevice, st);
     }
     // step t's end is kept from the last segment's start on
     const bool keep = t + 1 >= last0;
@@ -1434,10 +1440,13 @@ int cvr_adj_loss_grad(cvr_adj *a, int64_t nsteps, int64_t checkpoint_every, doub
   for (int64_t s = nseg - 1; s >= 0; --s) {
     const int64_t t0 = s * K, t1 = std::min(M, t0 + K);
     if (s < nseg - 1) {
-      const double *c = a->ck + (size_t)s * 3 * N3;
+      const double *c = a->ck + (size_t)s * ckn * N3;
       cudaMemcpyAsync(segX, c, B3, cudaMemcpyDeviceToDevice, st);
-      cudaMemcpyAsync(segF, c + N3, B3, cudaMemcpyDeviceToDevice, st);
-      cudaMemcpyAsync(a->V, c + 2 * N3, B3, cudaMemcpyDeviceToDevice, st);
+      cudaMemcpyAsync(a->V, c + N3, B3, cudaMemcpyDeviceToDevice, st);
+      if (ckn == 3)
+        cudaMemcpyAsync(segF, c + 2 * N3, B3, cudaMemcpyDeviceToDevice, st);
+      else if (int rc = eval_forces(a, segX, segF, 0.0))
+        return rc;
       for (int64_t t = t0; t < t1; ++t) {
         const int64_t q = t - t0;
         if (int rc = forward_step(a, segX + q * N3, segX + (q + 1) * N3, segF + q * N3, segF + (q + 1) * N3, 0.0))
