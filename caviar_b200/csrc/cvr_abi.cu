@@ -254,7 +254,10 @@ int dalloc(cvr_ctx *c, T **p, size_t count) {
   if (count == 0) count = 1;
   void *q = nullptr;
   cudaError_t e = cudaMalloc(&q, count * sizeof(T));
-  if (e != cudaSuccess) return fail(c, CVR_ERR_NOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+  if (e != cudaSuccess) {
+    cudaGetLastError();  // not the next launch's
+    return fail(c, CVR_ERR_NOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+  }
   cudaMemsetAsync(q, 0, count * sizeof(T), c->stream);
   c->all_allocs.push_back(q);
   *p = (T *)q;
@@ -1688,18 +1691,12 @@ int choose_tpa(const cvr_ctx *c, int64_t n) {
   return 1;
 }
 
-int ensure_ready(cvr_ctx *c) {
-  if (!c->have_state) return fail(c, CVR_ERR_STATE, "cvr_set_state has not been called");
-  if (!c->nl_set) return fail(c, CVR_ERR_STATE, "cvr_set_neighborlist has not been called");
-  return CVR_OK;
-}
-
-// Re-derive everything that depends on the settings (cells, tables, k-set).
 // Ewald self energy -(alpha / sqrt(pi)) k_e sum q^2 (electrostatic_ewald_k/energy.cpp:49).
 double self_energy(const cvr_ctx *c) {
   return c->ewk_on ? -0.56418958354775628695 * c->ewk_alpha * c->q2_sum * c->ewk_ke : 0.0;
 }
 
+// Re-derive everything that depends on the settings (cells, tables, k-set).
 int refresh(cvr_ctx *c) {
   if (!c->have_state || !c->nl_set) return CVR_OK;
   c->epoch++;  // settings may change what the step graphs bake in
@@ -1735,6 +1732,12 @@ int refresh(cvr_ctx *c) {
   c->list_fresh = false;
   c->setup_done = false;
   c->refreshed = true;
+  return CVR_OK;
+}
+
+int ensure_ready(cvr_ctx *c) {
+  if (!c->have_state) return fail(c, CVR_ERR_STATE, "cvr_set_state has not been called");
+  if (!c->nl_set) return fail(c, CVR_ERR_STATE, "cvr_set_neighborlist has not been called");
   return CVR_OK;
 }
 
@@ -2185,9 +2188,14 @@ int cvr_set_state(cvr_ctx *c, int64_t n, const double *pos, const double *vel, c
   if (c->all_atom && n > CVR_ALL_ATOM_MAX) return fail(c, CVR_ERR_INVALID, "all_atom_test is for small systems");
   cudaSetDevice(c->device);
   if (n != c->n || !c->x) {
-    c->refreshed = false;
-    if (int r = alloc_atoms(c, n)) return r;
-    if (int r = dalloc(c, &c->stage, 9 * (size_t)n)) return r;
+    // the arrays of the state so far go, whatever becomes of the new one
+    c->have_state = c->list_valid = c->refreshed = false;
+    int r = alloc_atoms(c, n);
+    if (!r) r = dalloc(c, &c->stage, 9 * (size_t)n);
+    if (r) {
+      c->n = 0;  // none of them counts
+      return r;
+    }
     c->cap = 0;
     c->tpa = choose_tpa(c, n);
     // list interleave: TPA lanes per atom, or quads of four entries when one lane per atom
