@@ -1700,7 +1700,7 @@ double self_energy(const cvr_ctx *c) {
 int refresh(cvr_ctx *c) {
   if (!c->have_state || !c->nl_set) return CVR_OK;
   c->epoch++;  // settings may change what the step graphs bake in
-  c->refreshed = false;
+  c->refreshed = c->list_valid = c->list_fresh = c->setup_done = false;
   c->e_self = self_energy(c);
   if (int r = setup_cells(c)) return r;
   if (int r = alloc_cells(c)) return r;
@@ -1728,9 +1728,6 @@ int refresh(cvr_ctx *c) {
     else
       set_smem_attrs<float>(c);
   }
-  c->list_valid = false;
-  c->list_fresh = false;
-  c->setup_done = false;
   c->refreshed = true;
   return CVR_OK;
 }
@@ -1738,7 +1735,8 @@ int refresh(cvr_ctx *c) {
 int ensure_ready(cvr_ctx *c) {
   if (!c->have_state) return fail(c, CVR_ERR_STATE, "cvr_set_state has not been called");
   if (!c->nl_set) return fail(c, CVR_ERR_STATE, "cvr_set_neighborlist has not been called");
-  return CVR_OK;
+  // settings that failed half way (too many cells, an allocation): the arrays are not theirs
+  return c->refreshed ? CVR_OK : refresh(c);
 }
 
 // all_atom_test: every owned pair (no shift) and every owned atom with every
