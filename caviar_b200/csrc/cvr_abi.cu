@@ -197,6 +197,7 @@ struct cvr_ctx {
   int sms = 148;
   void *x4b{};
   unsigned long long *step_ctrl{};
+  int *step_share{};
   double *step_part{}, *step_rec{}, *step_pos{};
   int step_launch = 0;
   unsigned barrier_polls = BARRIER_POLLS;
@@ -1008,6 +1009,14 @@ GridShape grid_shape(const cvr_ctx *c, int groups) {
   return g;
 }
 
+// Whether a grid that builds the list between its barriers has few enough
+// cells to scan and clear: a cell costs 0.14 us / threads there and next to
+// nothing in the staged build, whose kernels have a thread per cell, and whose
+// launches cost 20 us more (build call, one launch / staged: 500 atoms on 16,000
+// threads, 176,000 cells 53 / 74 us, 1.8 million 64 / 85; 100 atoms on 3200,
+// 389,000 cells 68 / 75).
+bool cells_fit(const cvr_ctx *c, const GridShape &g) { return c->ncells <= (int64_t)128 * g.grid * g.threads; }
+
 // Launches a kernel that meets at grid barriers.  The parity of its barrier
 // words moves on only when it was launched: it clears the next launch's pair.
 // LAUNCH_REFUSED where the driver will not hold the whole grid resident (part
@@ -1035,15 +1044,16 @@ int launch_cooperative(cvr_ctx *c, const void *kernel, const GridShape &g, void 
 // systems whose lists a warp per atom searches, else launch_build's.
 template <typename real>
 int launch_build_now(cvr_ctx *c, int count_only) {
-  if (c->timing || !c->cooperative || c->n > STEPS_MAX_ATOMS || list_kernel_kind(c) != CVR_LIST_WARP) {
+  const GridShape g = grid_shape(c, (int)c->n);
+  if (c->timing || !c->cooperative || c->n > STEPS_MAX_ATOMS || list_kernel_kind(c) != CVR_LIST_WARP ||
+      !cells_fit(c, g)) {
     launch_build<real>(c, count_only);
     return CVR_OK;
   }
   DevState<real> s = dev_state<real>(c);
-  const GridShape g = grid_shape(c, (int)c->n);
   const size_t smem = steps_smem(g.threads / 32);
   int log2_tpa = c->log2_tpa, launch = c->step_launch;
-  void *args[] = {&s, &c->step_ctrl, &launch, &c->barrier_polls, &count_only, &log2_tpa};
+  void *args[] = {&s, &c->step_ctrl, &c->step_share, &launch, &c->barrier_polls, &count_only, &log2_tpa};
   const int r = launch_cooperative(c, (const void *)k_build_once<real>, g, args, smem);
   if (r == LAUNCH_REFUSED) launch_build<real>(c, count_only);
   if (r != CVR_OK) return r == LAUNCH_REFUSED ? CVR_OK : r;
@@ -1087,6 +1097,7 @@ int read_flags(cvr_ctx *c, int out[4]) {
     cudaMemsetAsync(c->flags, 0, 4 * sizeof(int), c->stream);
     c->builds_seen = 0;
     cudaMemsetAsync(c->step_ctrl, 0, SC_WORDS * sizeof(unsigned long long), c->stream);
+    cudaMemsetAsync(c->step_share, 0, c->sms * sizeof(int), c->stream);
     cudaMemsetAsync(c->cell_count, 0, ((size_t)c->ncells + 1) * sizeof(int), c->stream);
     cudaMemsetAsync(c->cell_fill, 0, ((size_t)c->ncells + 1) * sizeof(int), c->stream);
     c->have_state = c->list_valid = c->setup_done = c->list_fresh = false;
@@ -1370,7 +1381,8 @@ bool steps_in_one(const cvr_ctx *c) {
   return c->use_graphs && !c->timing && c->cooperative && c->lj_on && !c->ewr_on && !(c->ewk_on && c->nk > 0) &&
          !c->all_atom &&
          c->integrator == 0 && !c->sc_on && !(c->ewk_on && c->dipole_mode) && c->n <= STEPS_MAX_ATOMS &&
-         (c->tpa == 32 || c->tpa == 8) && list_kernel_kind(c) == CVR_LIST_WARP;
+         (c->tpa == 32 || c->tpa == 8) && list_kernel_kind(c) == CVR_LIST_WARP &&
+         cells_fit(c, grid_shape(c, grid_for(c->n, 32 / c->tpa)));
 }
 
 template <typename real, int TPA, bool ONE_TYPE, bool FIXED>
@@ -1396,6 +1408,7 @@ int launch_steps_t(cvr_ctx *c, int nsteps, int64_t every, int64_t done) {
   a.by = a.bx + c->n;
   a.bz = a.by + c->n;
   a.ctrl = c->step_ctrl;
+  a.share_atoms = c->step_share;
   a.launch = c->step_launch;
   a.polls = c->barrier_polls;
   a.counters = c->counters;
@@ -1883,7 +1896,8 @@ int cvr_create(cvr_ctx **out, const double lo[3], const double hi[3], const int 
   }
   cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, device);
   if (cudaMallocHost(&c->back, sizeof(*c->back)) != cudaSuccess || dalloc(c, &c->flags, 6) != CVR_OK || dalloc(c, &c->counters, 2) != CVR_OK ||
-      dalloc(c, &c->step_ctrl, SC_WORDS) != CVR_OK || dalloc(c, &c->step_part, 4 * (size_t)c->sms) != CVR_OK ||
+      dalloc(c, &c->step_ctrl, SC_WORDS) != CVR_OK || dalloc(c, &c->step_share, (size_t)c->sms) != CVR_OK ||
+      dalloc(c, &c->step_part, 4 * (size_t)c->sms) != CVR_OK ||
       dalloc(c, &c->d_type_hist, MAX_TYPES + 1) != CVR_OK) {
     cudaEventDestroy(c->k_fork);
     cudaEventDestroy(c->k_join);

@@ -59,9 +59,9 @@ __device__ __forceinline__ void cell_xyz(const DevState<real> &s, int c, int &cx
 }
 
 // Pass 1: wrap (Domain::fix_position: one if / else-if per periodic axis),
-// cell index, copy the atom to the temporaries, count atoms per cell.
+// cell index (returned), copy the atom to the temporaries, count atoms per cell.
 template <typename real>
-__device__ __forceinline__ void bin_atom(const DevState<real> &s, int i) {
+__device__ __forceinline__ int bin_atom(const DevState<real> &s, int i) {
   double p[3] = {s.x[i], s.y[i], s.z[i]};
   int c[3];
   bool clamped = false;
@@ -93,6 +93,7 @@ __device__ __forceinline__ void bin_atom(const DevState<real> &s, int i) {
   s.tmol[i] = s.mol[i];
   s.tcell[i] = cell;
   atomicAdd(&s.cell_count[cell], 1);
+  return cell;
 }
 template <typename real>
 __global__ void k_bin_count(DevState<real> s) {
