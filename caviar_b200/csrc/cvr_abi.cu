@@ -1704,6 +1704,21 @@ int choose_tpa(const cvr_ctx *c, int64_t n) {
   return 1;
 }
 
+// Lanes per atom for the settings as they are; a change of lanes is a change
+// of the list's layout.  (Ewald terms set after the state: 8 lanes, chosen for
+// the LJ system before, against 32: 4500 ions FP64 102 / 86 us per step, 8000
+// FP64 131 / 115, mixed 74.4 / 70.6.  Langevin runs and single points of LJ
+// systems lose nothing with 8: 8000 atoms 29.9 us per step against 31.1 with 32.)
+void set_lanes(cvr_ctx *c) {
+  const int tpa = choose_tpa(c, c->n);
+  if (tpa == c->tpa && c->cap > 0) return;
+  c->tpa = tpa;
+  // list interleave: TPA lanes per atom, or quads of four entries when one lane per atom
+  c->log2_tpa = (c->tpa == 32) ? 5 : (c->tpa == 8 ? 3 : 2);
+  c->cap = 0;
+  c->epoch++;
+}
+
 // Ewald self energy -(alpha / sqrt(pi)) k_e sum q^2 (electrostatic_ewald_k/energy.cpp:49).
 double self_energy(const cvr_ctx *c) {
   return c->ewk_on ? -0.56418958354775628695 * c->ewk_alpha * c->q2_sum * c->ewk_ke : 0.0;
@@ -1714,6 +1729,7 @@ int refresh(cvr_ctx *c) {
   if (!c->have_state || !c->nl_set) return CVR_OK;
   c->epoch++;  // settings may change what the step graphs bake in
   c->refreshed = c->list_valid = c->list_fresh = c->setup_done = false;
+  set_lanes(c);
   c->e_self = self_energy(c);
   if (int r = setup_cells(c)) return r;
   if (int r = alloc_cells(c)) return r;
@@ -2209,9 +2225,7 @@ int cvr_set_state(cvr_ctx *c, int64_t n, const double *pos, const double *vel, c
       return r;
     }
     c->cap = 0;
-    c->tpa = choose_tpa(c, n);
-    // list interleave: TPA lanes per atom, or quads of four entries when one lane per atom
-    c->log2_tpa = (c->tpa == 32) ? 5 : (c->tpa == 8 ? 3 : 2);
+    set_lanes(c);
   }
   // The types first, then the atoms per type on the GPU (the range check of
   // every type, and the charge and mass sums at one term per type): the
