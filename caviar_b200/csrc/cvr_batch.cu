@@ -59,15 +59,24 @@ struct KRunB {
   int nx, ny, nz0, len, k0, skip;
 };
 
-// LJ pair lists of the larger replicas: entries per atom, skin as a fraction
-// of the LJ cutoff, and the smallest replica that uses one.  With all pairs,
-// three tiles in four hold no charged pair and test 32 x 32 atoms for the few
-// per cent within the LJ cutoff.  50 steps of 296 equal replicas, all pairs ->
-// list: 5.51 -> 5.67 ms at 150 atoms, 7.20 -> 6.53 at 200, 12.4 -> 11.5 at 400,
-// 24.6 -> 19.0 at 600; 1024 replicas of 64-2048 atoms, 20 steps: 83.7 -> 57.5 ms.
+// LJ pair lists: entries per atom, skin as a fraction of the LJ cutoff, and
+// which replicas have one.  With all pairs, the tiles without a charged pair
+// test 32 x 32 atoms for the few per cent within the LJ cutoff.  Per 20 steps,
+// half the atoms charged, all pairs -> list: 296 replicas of 200 atoms 1.91 ->
+// 1.66 ms, 600 7.55 -> 5.34; 148 of 1500 15.5 -> 9.26; 1024 of 64-2048 atoms
+// 83.7 -> 56 (150 atoms would lose 3 %).  A list pays
+//  * from LIST_MIN atoms;
+//  * where its rows fit LCAP: at most LIST_MEAN_MAX expected partners (fluids
+//    stay within about 15 of the mean).  Beyond that it would be built and
+//    thrown away (cutoff 3 at density 0.8, 600 atoms: 8.49 ms, all pairs 7.63);
+//  * where the charged atoms, whose tiles run in any case, are at most
+//    LIST_NQ_MAX of all (all of them charged: 22.2 ms at 1500 atoms, all pairs
+//    21.0; 600 atoms 11.0 and 10.3).
 constexpr int LCAP = 128;
 constexpr double LSKIN = 0.12;
 constexpr int LIST_MIN = 192;
+constexpr double LIST_MEAN_MAX = 110.0;
+constexpr double LIST_NQ_MAX = 0.7;
 
 constexpr int KFILL_MASK = (1 << 30) - 1;
 constexpr int KTWICE = 1 << 30;
@@ -86,14 +95,16 @@ struct BatchDev {
   // filled from it), bit 30 = k's force term counts twice (its mirror is skipped)
   const int *kinfo;
   double *out;  // [replica][NTH]
-  // LJ lists: of replica r, entry k of atom i at list[LCAP * off[r] + k * n + i];
-  // neighbours per atom; coordinates at the build, SoA [3][atoms]; per replica
-  // whether its list is in use (carried between launches, as the forces are)
+  // LJ lists: replica r's begins at atom loff[r] of the listed ones (-1: it
+  // has none); entry k of atom i at list[LCAP * loff[r] + k * n + i];
+  // neighbours per atom; coordinates at the build, [3][n] per replica; per
+  // replica whether its list is in use (carried between launches, as the
+  // forces are)
+  const long long *loff;
   uint16_t *list;
   int *list_count;
   uint32_t *list_u;
   int *list_on;
-  long long n_total;
   int nk, nruns, kmax, n_types;
   float eps[TMAX * TMAX], sig[TMAX * TMAX], charge[TMAX];
   double mass[TMAX], mass_inv[TMAX], chargeD[TMAX];
@@ -296,8 +307,9 @@ __device__ __forceinline__ void tile_diag(const Smem &S, const PairK &K, int I, 
 // less than one; rl2 is widened for that): converting three differences to
 // float would keep the conversion unit busy for twice the test's issue slots.
 template <int TPB>
-__device__ bool build_lj_list(const BatchDev &p, const Smem &S, int n, long long o, int rl2) {
-  uint16_t *list = p.list + (size_t)LCAP * o;
+__device__ bool build_lj_list(const BatchDev &p, const Smem &S, int n, long long lo, int rl2) {
+  uint16_t *list = p.list + (size_t)LCAP * lo;
+  uint32_t *u = p.list_u + 3 * lo;
   bool over = false;
   for (int i = threadIdx.x; i < n; i += TPB) {
     const float4 ih = S.xh[i];
@@ -314,10 +326,10 @@ __device__ bool build_lj_list(const BatchDev &p, const Smem &S, int n, long long
       }
     }
     over = over || cnt > LCAP;
-    p.list_count[o + i] = min(cnt, LCAP);
-    p.list_u[o + i] = ux;
-    p.list_u[p.n_total + o + i] = uy;
-    p.list_u[2 * p.n_total + o + i] = uz;
+    p.list_count[lo + i] = min(cnt, LCAP);
+    u[i] = ux;
+    u[n + i] = uy;
+    u[2 * n + i] = uz;
   }
   return !__syncthreads_or(over);
 }
@@ -325,12 +337,12 @@ __device__ bool build_lj_list(const BatchDev &p, const Smem &S, int n, long long
 // LJ forces from the list, each thread its own atoms, added to S.fs* (units
 // of h); energies and virial into e as pair_c (both ends: weight 1/2).
 template <int TPB, bool UNI, bool EV>
-__device__ __forceinline__ void lj_list(const BatchDev &p, const Smem &S, const PairK &K, int n, long long o,
+__device__ __forceinline__ void lj_list(const BatchDev &p, const Smem &S, const PairK &K, int n, long long lo,
                                         double (&e)[3]) {
   for (int i = threadIdx.x; i < n; i += TPB) {
     const float4 ih = S.xh[i], none = make_float4(0.f, 0.f, 0.f, 0.f);
-    const uint16_t *row = p.list + (size_t)LCAP * o + i;
-    const int cnt = p.list_count[o + i];
+    const uint16_t *row = p.list + (size_t)LCAP * lo + i;
+    const int cnt = p.list_count[lo + i];
     float f[3] = {0.f, 0.f, 0.f};
     for (int k = 0; k < cnt; k += 4) {
       int j[4];
@@ -354,9 +366,10 @@ __device__ __forceinline__ void lj_list(const BatchDev &p, const Smem &S, const 
 // Forces of the replica's current positions into S.fs* (all pairs under the
 // minimum image, then k space).  EV: energies and virial into ev[0..4]
 // (this thread's share: lj, ewald_r, ewald_k, -, virial).
-template <int TPB, bool UNI, bool EV>
-__device__ void batch_forces(const BatchDev &p, const Smem &S, int r, int n, int nq, double L, int G, bool listed,
+template <int TPB, bool UNI, bool EV, bool LIST>
+__device__ void batch_forces(const BatchDev &p, const Smem &S, int r, int n, int nq, double L, int G, bool list_on,
                              double (&ev)[5]) {
+  const bool listed = LIST && list_on;
   constexpr int W = TPB / 32;
   const int warp = threadIdx.x >> 5;
   const double h = L * 2.3283064365386963e-10;  // L / 2^32
@@ -409,7 +422,7 @@ __device__ void batch_forces(const BatchDev &p, const Smem &S, int r, int n, int
   }
   __syncthreads();
   if (listed) {
-    lj_list<TPB, UNI, EV>(p, S, K, n, p.off[r], e);
+    lj_list<TPB, UNI, EV>(p, S, K, n, p.loff[r], e);
     __syncthreads();
   }
   // pair forces from units of h back to length units
@@ -569,12 +582,15 @@ __device__ __forceinline__ void to_smem(const BatchDev &p, const Smem &S, int i,
 // whether energies are wanted).  Each thread owns atoms tid, tid + TPB, ...
 // for the integrator and the k-space force; the pair tiles write forces of
 // any atom, ordered by barriers.
-template <int TPB, bool UNI>
+// LIST: for the replicas with an LJ list, the others' blocks return at once (in
+// one kernel for both, replicas of all pairs took 1-3 % longer).
+template <int TPB, bool UNI, bool LIST>
 __global__ void __launch_bounds__(TPB, 1) k_batch(BatchDev p, int first, int nsteps, int np, int G,
                                                    int compute_first) {
   extern __shared__ __align__(16) unsigned char smraw[];
   const int r = p.order[first + blockIdx.x];
   const int n = p.n[r], nq = p.nq[r];
+  if ((p.loff[r] >= 0 && nq <= LIST_NQ_MAX * n) != LIST) return;
   const long long o = p.off[r];
   const double L = p.L[r];
   const Smem S = carve(smraw, p.nk, np, G);
@@ -610,23 +626,23 @@ __global__ void __launch_bounds__(TPB, 1) k_batch(BatchDev p, int first, int nst
     }
   }
   __syncthreads();
-  // the LJ list (larger replicas): rebuilt when an atom has moved half the
-  // skin since the build (a little less, for the rounding of the test)
-  const bool wants_list = n >= LIST_MIN;
+  double ev[5] = {0, 0, 0, 0, 0};
+  // the LJ list: rebuilt when an atom has moved half the skin since the build
+  // (a little less, for the rounding of the test)
+  const long long lo = p.loff[r];
   int rl2 = 0;
   float moved2 = 0.f;
   bool listed = false;
-  if (wants_list) {
+  if (LIST) {
     // below (0.56 x 2^15 + 1.8)^2 < 2^31: the cutoff is at most half the box
-    const double rl = p.rc_lj[r] * (1.0 + LSKIN) * 32768.0 / L + 1.7320508075688774;
+    const double rl = fabs(p.rc_lj[r]) * (1.0 + LSKIN) * 32768.0 / L + 1.7320508075688774;
     const double half = 0.4999 * p.rc_lj[r] * LSKIN * 4294967296.0 / L;
     rl2 = (int)ceil(rl * rl);
     moved2 = (float)(half * half);
-    listed = compute_first ? build_lj_list<TPB>(p, S, n, o, rl2) : p.list_on[r] != 0;
+    listed = compute_first ? build_lj_list<TPB>(p, S, n, lo, rl2) : p.list_on[r] != 0;
   }
-  double ev[5] = {0, 0, 0, 0, 0};
   if (compute_first) {
-    batch_forces<TPB, UNI, false>(p, S, r, n, nq, L, G, listed, ev);
+    batch_forces<TPB, UNI, false, LIST>(p, S, r, n, nq, L, G, listed, ev);
   } else {
     for (int i = threadIdx.x; i < n; i += TPB) {
       S.fsx[i] = p.fx[o + i];
@@ -652,16 +668,20 @@ __global__ void __launch_bounds__(TPB, 1) k_batch(BatchDev p, int first, int nst
         X[a][gi] = x;
       }
       to_smem(p, S, i, gi, L);
-      if (listed) {
+      if (LIST && listed) {
         const float4 u = S.xh[i];
-        const float dx = (float)(int)(__float_as_uint(u.x) - p.list_u[gi]),
-                    dy = (float)(int)(__float_as_uint(u.y) - p.list_u[p.n_total + gi]),
-                    dz = (float)(int)(__float_as_uint(u.z) - p.list_u[2 * p.n_total + gi]);
+        const uint32_t *b = p.list_u + 3 * lo + i;
+        const float dx = (float)(int)(__float_as_uint(u.x) - b[0]), dy = (float)(int)(__float_as_uint(u.y) - b[n]),
+                    dz = (float)(int)(__float_as_uint(u.z) - b[2 * n]);
         moved = moved || !(dx * dx + dy * dy + dz * dz <= moved2);
       }
     }
-    if (__syncthreads_or(moved)) listed = build_lj_list<TPB>(p, S, n, o, rl2);
-    batch_forces<TPB, UNI, false>(p, S, r, n, nq, L, G, listed, ev);
+    if (LIST) {
+      if (__syncthreads_or(moved)) listed = build_lj_list<TPB>(p, S, n, lo, rl2);
+    } else {
+      __syncthreads();
+    }
+    batch_forces<TPB, UNI, false, LIST>(p, S, r, n, nq, L, G, listed, ev);
     for (int i = threadIdx.x; i < n; i += TPB) {
       const long long gi = o + i;
       const double mi = p.mass_inv[p.type[gi]];
@@ -671,14 +691,14 @@ __global__ void __launch_bounds__(TPB, 1) k_batch(BatchDev p, int first, int nst
     }
   }
   // forces of the final positions and the list's state, carried to the next launch
-  if (wants_list && threadIdx.x == 0) p.list_on[r] = listed;
+  if (LIST && threadIdx.x == 0) p.list_on[r] = listed;
   for (int i = threadIdx.x; i < n; i += TPB) {
     p.fx[o + i] = S.fsx[i];
     p.fy[o + i] = S.fsy[i];
     p.fz[o + i] = S.fsz[i];
   }
   __syncthreads();
-  batch_forces<TPB, UNI, true>(p, S, r, n, nq, L, G, listed, ev);  // energies only; S.fs* is scratch here
+  batch_forces<TPB, UNI, true, LIST>(p, S, r, n, nq, L, G, listed, ev);  // energies only; S.fs* is scratch here
   __syncthreads();
   // kinetic energy (COM removed), energies
   double kv[9] = {0, 0, 0, 0, 0, ev[0], ev[1], ev[4], ev[2]};
@@ -805,15 +825,14 @@ using KernelFn = void (*)(BatchDev, int, int, int, int, int);
 
 struct Shape {
   int tpb;
-  KernelFn fn, fn_uni;
+  KernelFn fn[2][2];  // [uniform LJ][list]
 };
 
 // Launch shapes (threads per CTA); the uniform-LJ form when every type pair has the same eps and sigma
-const Shape kShapes[] = {
-    {128, k_batch<128, false>, k_batch<128, true>},
-    {256, k_batch<256, false>, k_batch<256, true>},
-    {512, k_batch<512, false>, k_batch<512, true>},
-};
+template <int TPB> constexpr Shape shape_of() {
+  return {TPB, {{k_batch<TPB, false, false>, k_batch<TPB, false, true>}, {k_batch<TPB, true, false>, k_batch<TPB, true, true>}}};
+}
+const Shape kShapes[] = {shape_of<128>(), shape_of<256>(), shape_of<512>()};
 
 }  // namespace
 
@@ -825,6 +844,7 @@ struct cvr_batch {
   std::vector<int> n;
   std::vector<long long> off;
   std::vector<double> L, rc_lj, rc_r;
+  std::vector<int> order;    // replicas in decreasing size
   int *slot_of = nullptr;    // device: caller's atom index -> stored slot (charged atoms first within a replica)
   double *stage = nullptr;   // device: 9 doubles per atom, the caller's layout
   int *stage_type = nullptr; // device, and one counter behind it
@@ -832,13 +852,17 @@ struct cvr_batch {
   bool uniform = false;      // every type pair has the same eps and sigma
   BatchDev dev{};
   std::vector<void *> allocs;
+  void *list_mem = nullptr;  // LJ lists of list_atoms atoms
+  long long list_atoms = 0;
   // size classes: [first, count) in the order array, chosen shape
   struct Class {
     int first, count, nmax, shape;
+    bool lists;  // whether a replica of the class may have an LJ list
   };
   std::vector<Class> classes;
-  cudaStream_t side[3] = {nullptr, nullptr, nullptr};  // one per size class: the graph's parallel branches
-  cudaEvent_t fork = nullptr, join[3] = {nullptr, nullptr, nullptr};
+  // the graph's parallel branches, two per size class (without and with LJ lists)
+  cudaStream_t side[6] = {};
+  cudaEvent_t fork = nullptr, join[6] = {};
   // one graph per (nsteps, forces of the first positions computed in the launch)
   cudaGraphExec_t graph[2] = {nullptr, nullptr};
   int graph_steps[2] = {-1, -1};
@@ -864,13 +888,50 @@ int balloc(cvr_batch *b, T **p, size_t count) {
   return CVR_OK;
 }
 
-int launch_class(cvr_batch *b, const cvr_batch::Class &c, int shape, int nsteps, int compute_first,
+// Which replicas have an LJ list, and room for those (none where memory does
+// not hold them: all pairs then).
+int place_lists(cvr_batch *b) {
+  std::vector<long long> loff(b->n_rep, -1);
+  long long atoms = 0;
+  for (int r = 0; r < b->n_rep; ++r) {
+    const double rl = std::fabs(b->rc_lj[r]) * (1.0 + LSKIN) / b->L[r];
+    if (b->n[r] < LIST_MIN || !(4.18879 * rl * rl * rl * b->n[r] <= LIST_MEAN_MAX)) continue;
+    loff[r] = atoms;
+    atoms += b->n[r];
+  }
+  if (atoms > b->list_atoms) {
+    if (b->list_mem) cudaFree(b->list_mem);
+    b->list_mem = nullptr;
+    b->list_atoms = 0;
+    const size_t per_atom = LCAP * sizeof(uint16_t) + sizeof(int) + 3 * sizeof(uint32_t);
+    if (cudaMalloc(&b->list_mem, atoms * per_atom) == cudaSuccess) {
+      b->list_atoms = atoms;
+      b->dev.list = static_cast<uint16_t *>(b->list_mem);
+      b->dev.list_count = reinterpret_cast<int *>(b->dev.list + (size_t)LCAP * atoms);
+      b->dev.list_u = reinterpret_cast<uint32_t *>(b->dev.list_count + atoms);
+    } else {
+      cudaGetLastError();
+      b->list_mem = nullptr;
+      std::fill(loff.begin(), loff.end(), -1);
+    }
+  }
+  for (cvr_batch::Class &c : b->classes) {
+    c.lists = false;
+    for (int k = c.first; k < c.first + c.count; ++k) c.lists = c.lists || loff[b->order[k]] >= 0;
+  }
+  if (cudaMemcpy(const_cast<long long *>(b->dev.loff), loff.data(), b->n_rep * sizeof(long long),
+                 cudaMemcpyHostToDevice) != cudaSuccess)
+    return bfail(b, CVR_ERR_CUDA, "list offsets");
+  return CVR_OK;
+}
+
+int launch_class(cvr_batch *b, const cvr_batch::Class &c, int shape, int nsteps, int compute_first, int list,
                  cudaStream_t st) {
   const Shape &s = kShapes[shape];
   const int np = (c.nmax + 31) & ~31;
   const int G = groups_for(s.tpb, b->dev.nruns);
-  (b->uniform ? s.fn_uni : s.fn)<<<c.count, s.tpb, smem_bytes(b->dev.nk, np, G), st>>>(b->dev, c.first, nsteps, np,
-                                                                                         G, compute_first);
+  s.fn[b->uniform][list]<<<c.count, s.tpb, smem_bytes(b->dev.nk, np, G), st>>>(b->dev, c.first, nsteps, np, G,
+                                                                              compute_first);
   return cudaGetLastError() == cudaSuccess ? CVR_OK : CVR_ERR_CUDA;
 }
 
@@ -901,7 +962,7 @@ int cvr_batch_create(cvr_batch **out, int n_rep, const int64_t *n_atoms, const d
   b->n_total = o;
   cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking);
   cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming);
-  for (int c = 0; c < 3; ++c) {
+  for (int c = 0; c < 6; ++c) {
     cudaStreamCreateWithFlags(&b->side[c], cudaStreamNonBlocking);
     cudaEventCreateWithFlags(&b->join[c], cudaEventDisableTiming);
   }
@@ -938,12 +999,9 @@ int cvr_batch_create(cvr_batch **out, int n_rep, const int64_t *n_atoms, const d
   d.vz = arr + 5 * N;
   cudaMemset(farr, 0, 3 * N * sizeof(float));
   cudaMemset(dtype, 0, N * sizeof(int));
-  uint16_t *list;
-  if ((rc = balloc(b, &list, (size_t)LCAP * N)) || (rc = balloc(b, &d.list_count, N)) || (rc = balloc(b, &d.list_u, 3 * N)) ||
-      (rc = balloc(b, &d.list_on, n_rep)))
-    return rc;
-  d.list = list;
-  d.n_total = o;
+  long long *loff;
+  if ((rc = balloc(b, &loff, n_rep)) || (rc = balloc(b, &d.list_on, n_rep))) return rc;
+  d.loff = loff;
   d.fx = farr;
   d.fy = farr + N;
   d.fz = farr + 2 * N;
@@ -957,7 +1015,8 @@ int cvr_batch_create(cvr_batch **out, int n_rep, const int64_t *n_atoms, const d
   d.rc_lj = dL + n_rep;
   d.rc_r = dL + 2 * n_rep;
   // replicas in decreasing size; size classes by the atoms-per-thread a shape needs
-  std::vector<int> order(n_rep);
+  std::vector<int> &order = b->order;
+  order.resize(n_rep);
   for (int r = 0; r < n_rep; ++r) order[r] = r;
   std::stable_sort(order.begin(), order.end(), [&](int a, int c) { return b->n[a] > b->n[c]; });
   const int bounds[3] = {2048, 1024, 512};
@@ -966,7 +1025,7 @@ int cvr_batch_create(cvr_batch **out, int n_rep, const int64_t *n_atoms, const d
     const int hi = bounds[ci], lo = (ci < 2) ? bounds[ci + 1] : 0;
     const int first = k;
     while (k < n_rep && b->n[order[k]] > lo && b->n[order[k]] <= hi) ++k;
-    if (k > first) b->classes.push_back({first, k - first, b->n[order[first]], -1});
+    if (k > first) b->classes.push_back({first, k - first, b->n[order[first]], -1, false});
   }
   cudaMemcpy(dn, b->n.data(), n_rep * sizeof(int), cudaMemcpyHostToDevice);
   cudaMemset(dn + n_rep, 0, n_rep * sizeof(int));
@@ -984,7 +1043,8 @@ void cvr_batch_destroy(cvr_batch *b) {
   for (cudaGraphExec_t g : b->graph)
     if (g) cudaGraphExecDestroy(g);
   for (void *p : b->allocs) cudaFree(p);
-  for (int c = 0; c < 3; ++c) {
+  if (b->list_mem) cudaFree(b->list_mem);
+  for (int c = 0; c < 6; ++c) {
     cudaStreamDestroy(b->side[c]);
     cudaEventDestroy(b->join[c]);
   }
@@ -1013,6 +1073,7 @@ int cvr_batch_set_forces(cvr_batch *b, const double *eps, const double *sigma, c
   b->rc_r.assign(rc_r, rc_r + b->n_rep);
   cudaMemcpy((void *)b->dev.rc_lj, rc_lj, b->n_rep * sizeof(double), cudaMemcpyHostToDevice);
   cudaMemcpy((void *)b->dev.rc_r, rc_r, b->n_rep * sizeof(double), cudaMemcpyHostToDevice);
+  if (int rc = place_lists(b)) return rc;
   b->dev.alpha = alpha;
   b->dev.k_e = k_e;
   b->dev.dt = dt;
@@ -1072,9 +1133,10 @@ int cvr_batch_set_forces(cvr_batch *b, const double *eps, const double *sigma, c
   b->dev.kinfo = dki;
   for (const Shape &s : kShapes) {
     const int sm = (int)smem_bytes(b->dev.nk, NMAX, groups_for(s.tpb, b->dev.nruns));
-    if (cudaFuncSetAttribute(s.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, sm) != cudaSuccess ||
-        cudaFuncSetAttribute(s.fn_uni, cudaFuncAttributeMaxDynamicSharedMemorySize, sm) != cudaSuccess)
-      return bfail(b, CVR_ERR_CUDA, "shared memory attribute");
+    for (const auto &fns : s.fn)
+      for (KernelFn fn : fns)
+        if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, sm) != cudaSuccess)
+          return bfail(b, CVR_ERR_CUDA, "shared memory attribute");
   }
   b->tuned = false;
   b->forces_valid = false;
@@ -1131,7 +1193,7 @@ static int batch_tune(cvr_batch *b) {
       if (smem_bytes(b->dev.nk, np, groups_for(s.tpb, b->dev.nruns)) > 227 * 1024) continue;
       if (s.tpb > 2 * np) continue;  // more threads than pair-tile warps and atoms can use
       cudaEventRecord(e0, b->stream);
-      if (launch_class(b, c, si, 2, 1, b->stream)) {
+      if (launch_class(b, c, si, 2, 1, 0, b->stream) || (c.lists && launch_class(b, c, si, 2, 1, 1, b->stream))) {
         cudaFree(save);
         return bfail(b, CVR_ERR_CUDA, "tuning launch failed");
       }
@@ -1182,12 +1244,14 @@ int cvr_batch_run(cvr_batch *b, int64_t nsteps, double *out) {
     // SMs the large-replica class leaves idle
     int lrc = CVR_OK;
     cudaEventRecord(b->fork, b->stream);
-    for (size_t ci = 0; ci < b->classes.size(); ++ci) {
-      cudaStreamWaitEvent(b->side[ci], b->fork, 0);
-      lrc |= launch_class(b, b->classes[ci], b->classes[ci].shape, (int)nsteps, first, b->side[ci]);
-      cudaEventRecord(b->join[ci], b->side[ci]);
-      cudaStreamWaitEvent(b->stream, b->join[ci], 0);
-    }
+    for (size_t ci = 0; ci < b->classes.size(); ++ci)
+      for (int list = b->classes[ci].lists; list >= 0; --list) {
+        const size_t k = 2 * ci + list;
+        cudaStreamWaitEvent(b->side[k], b->fork, 0);
+        lrc |= launch_class(b, b->classes[ci], b->classes[ci].shape, (int)nsteps, first, list, b->side[k]);
+        cudaEventRecord(b->join[k], b->side[k]);
+        cudaStreamWaitEvent(b->stream, b->join[k], 0);
+      }
     const cudaError_t ce = cudaStreamEndCapture(b->stream, &g);
     if (ce != cudaSuccess || lrc != CVR_OK) return bfail(b, CVR_ERR_CUDA, "capture of the replica launches failed");
     if (cudaGraphInstantiate(&graph, g, 0) != cudaSuccess) return bfail(b, CVR_ERR_CUDA, "instantiate");
