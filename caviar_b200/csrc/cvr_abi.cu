@@ -1574,7 +1574,7 @@ int run_impl(cvr_ctx *c, int64_t nsteps, int64_t every, double *thermo) {
     }
     int64_t k0 = 0;  // steps done in launches of many
     while (graphs && k0 < nsteps && steps_in_one(c)) {
-      const int chunk = (int)std::min<int64_t>(nsteps - k0, STEPS_MAX);
+      const int chunk = (int)std::min({nsteps - k0, (int64_t)STEPS_MAX, STEPS_ATOMS_MAX / c->n});
       const int r = launch_steps<real>(c, chunk, every, k0);
       if (r == CVR_OK) k0 += chunk;
       else if (r != LAUNCH_REFUSED) return r;

@@ -69,7 +69,12 @@ template <typename real> struct StepArgs {
 };
 
 constexpr unsigned BARRIER_POLLS = 1u << 22;  // a barrier's wait: some seconds
-constexpr int STEPS_MAX = 1 << 16;            // steps per launch (the need field's range)
+// Steps per launch (the need field holds 2^24 / 148 of them).  The blocks hold
+// their SMs for the whole launch, and other streams wait that long: at most
+// about 15 ms (1024 steps of 500 atoms 6.2 ms, of 16,000 13-16; 256 of 65,000
+// 10-12), which the 10 us of a launch do not lengthen (0.2 %).
+constexpr int STEPS_MAX = 1024;
+constexpr int64_t STEPS_ATOMS_MAX = 1 << 24;  // steps x atoms
 
 // Grid barrier on a counter per parity of the barrier: every block adds 1,
 // plus 2^32 if it asks for a list rebuild and 2^56 if it met an error, and
