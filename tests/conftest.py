@@ -13,6 +13,13 @@ def pytest_configure(config):
     config.addinivalue_line("markers", "reference: needs the reference harness built from the reference sources")
 
 
+def pytest_collection_modifyitems(items):
+    # test_integration.py runs a binary built from the reference's sources and
+    # fails where that could not be built: after all the others, so that a run
+    # that stops at the first failure has run them
+    items.sort(key=lambda item: item.path.name == "test_integration.py")
+
+
 @pytest.fixture(scope="session")
 def oracle_lib():
     from oracle import oracle as O
