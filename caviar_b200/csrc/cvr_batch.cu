@@ -1073,6 +1073,13 @@ int cvr_batch_set_forces(cvr_batch *b, const double *eps, const double *sigma, c
   b->rc_r.assign(rc_r, rc_r + b->n_rep);
   cudaMemcpy((void *)b->dev.rc_lj, rc_lj, b->n_rep * sizeof(double), cudaMemcpyHostToDevice);
   cudaMemcpy((void *)b->dev.rc_r, rc_r, b->n_rep * sizeof(double), cudaMemcpyHostToDevice);
+  // the graphs hold the lists' addresses
+  for (cudaGraphExec_t &g : b->graph)
+    if (g) {
+      cudaGraphExecDestroy(g);
+      g = nullptr;
+    }
+  b->tuned = b->forces_valid = false;
   if (int rc = place_lists(b)) return rc;
   b->dev.alpha = alpha;
   b->dev.k_e = k_e;
@@ -1138,13 +1145,6 @@ int cvr_batch_set_forces(cvr_batch *b, const double *eps, const double *sigma, c
         if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, sm) != cudaSuccess)
           return bfail(b, CVR_ERR_CUDA, "shared memory attribute");
   }
-  b->tuned = false;
-  b->forces_valid = false;
-  for (cudaGraphExec_t &g : b->graph)
-    if (g) {
-      cudaGraphExecDestroy(g);
-      g = nullptr;
-    }
   return CVR_OK;
 }
 
