@@ -42,9 +42,11 @@ constexpr int KMZ = 16;    // k-force: Z[m] held in registers up to this many m-
 #endif
 constexpr int KF_WMAX = CVR_KF_WMAX;  // k-force: most warps per block of 32 atoms
 constexpr int KRW = 16;    // warps of the S(k) chunk reduction
-// Many steps in one launch (k_steps) up to this many atoms, the range of the
-// warp-per-atom list search (per step, one kernel per stage -> k_steps: 20.5 ->
-// 7.0 us at 500 LJ atoms, 50.1 -> 40.7 at 65,001).
+// Many steps in one launch (k_steps) up to this many atoms, and the automatic
+// choice of the warp-per-atom list search, which k_steps uses.  Not where
+// k_steps stops winning: 62,500 LJ atoms, one kernel per stage with the thread
+// search -> k_steps, 43.1 -> 40.1 us per step mixed, 55.3 -> 48.9 FP64; above,
+// only the staged path was measured.
 constexpr int64_t STEPS_MAX_ATOMS = 65536;
 constexpr size_t KF_COEF_SMEM = 72 * 1024;  // k-force: shared memory for staged column coefficients
 
@@ -680,8 +682,9 @@ int alloc_list(cvr_ctx *c, int cap) {
 
 // ------------------------------------------------------------- launches
 // The list search kernel: by default systems up to 65,536 atoms take the
-// warp kernel, larger ones one thread per atom (LJ fluid, mixed step: warp
-// 34.2 vs thread 38.5 us at 32,000 atoms, 59.5 vs 50.7 us at 108,000).
+// warp kernel, larger ones one thread per atom (LJ fluid, mixed, a whole staged
+// build, warp / thread: 93 / 115 us at 32,000 atoms, 141 / 132 at 62,500, 211 /
+// 153 at 108,000; up to 65,536 the warp search brings k_steps with it).
 int list_kernel_kind(const cvr_ctx *c) {
   if (c->list_kernel != CVR_LIST_AUTO) return c->list_kernel;
   return (c->n <= STEPS_MAX_ATOMS) ? CVR_LIST_WARP : CVR_LIST_THREAD;

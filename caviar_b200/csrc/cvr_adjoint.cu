@@ -194,7 +194,7 @@ __global__ void __launch_bounds__(256) k_adj_prep(Params p, PrepArgs a, typename
 // sums.  part[((chunk*NV + v)*M + m)*ncol + col], v = S+, S-, (T+, T-).
 // Latency-bound at 4000 atoms (two blocks per SM): SK_MG and the stage are
 // small to spread the sums.  One thread per k-vector over 256 atoms took 73 us
-// (VJP 145; FP64 VJP at 1372 atoms 196); now 8.9, 12.8 and 12.6.
+// (VJP 145; FP64 VJP at 1372 atoms 196); now 10, 14 and 14.
 template <typename real, bool VJP>
 __global__ void __launch_bounds__(SK_THREADS) k_adj_sk(Params p, const typename R2<real>::t *__restrict__ tab,
                                                        const double *__restrict__ U, int chunk, int nch0,
@@ -529,11 +529,13 @@ __device__ __forceinline__ real apply(real c, real c1, const real (&d)[3], const
 // evaluated 32 at a time, so the long terms run with full warps.  Partners of
 // one species at a time: the type pair is uniform and its constants and sums
 // are fixed registers.  Two partners per lane and round keep two loads in
-// flight and halve the loop's own cost (mixed; 68 -> 52 us for the energy
-// form at 4000 atoms, rc 8).  Issue bound (76 % of the slots; FP64: its
-// pipe).  4000 atoms, rc 8, mixed, with every lane evaluating its own partner
-// under divergence and FP64 differences: 216 us energy form with k space, 270
-// VJP; now 52 and 64 (+ 10 and 14 for the k-space kernel).
+// flight and halve the loop's own cost (68 -> 52 us for the energy form at
+// 4000 atoms, rc 8, before the exact displacements, which took it to 58).
+// Issue bound, mixed (77 % of the slots, 41 % of the warps); FP64 54 % at 22 %
+// of the warps, its pipe 37 %.  4000 atoms, rc 8, mixed, with every lane
+// evaluating its own partner under divergence and FP64 differences: 216 us
+// energy form with k space, 270 VJP; now 58 and 69 (+ 11 and 15 for the
+// k-space kernel).
 template <typename real, typename Coord, bool VJP>
 __global__ void __launch_bounds__(PAIR_WARPS * 32, Coord::MIN_BLOCKS)
     k_adj_pair(Params p, PairC<real> pc, const double *__restrict__ X, const double *__restrict__ U,

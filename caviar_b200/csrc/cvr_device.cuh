@@ -120,8 +120,11 @@ __device__ __forceinline__ float erfc_as(float x, float ex) {
 // exp(x^2) erfc(x) comes out within 6.5e-16 relative on [0, 12].  Even and odd
 // powers in two chains, no branches: the four pairs a lane has in flight
 // interleave, which the library function's branches prevent.  8000 ions, pair
-// kernel alone: 76.4 us with the library's erfc (FP64 pipe 43 % busy), 56.5
-// with this; trajectory adjoint at 1372 atoms 38.8 -> 34.0.
+// kernel alone: 76.4 us with the library's erfc, 56.5 with this (FP64 pipe 45 %
+// busy, 27 % of the warps); trajectory adjoint at 1372 atoms 38.8 -> 32-34.  ex
+// carries the rounding of its own argument (2 x^2 2^-53 relative), which the
+// force term beside it has too: total forces of 8000 ions are 5.3e-14 from 64-bit
+// sums with either erfc.
 __device__ __forceinline__ double erfc_ex(double x, double ex) {
   const double a = x + 3.75, b = fma(2.0, x, 1.0);
   const double r = 1.0 / (a * b);

@@ -94,7 +94,7 @@ __device__ __forceinline__ double2 phase(double u, int m) {
 // operations, against 4096 x 12 with one thread per k-vector.  20001 atoms,
 // k_max 8, whole call: 172 -> 32.8 us (100,000 atoms: 37 us at k_max 4, 209
 // at 10).  Two columns per thread (half the reads of Z): 31.9, 41 and 215 us,
-// so the reads are not what bounds it; the FP64 pipe is 40 % busy, the rest
+// so the reads are not what bounds it; the FP64 pipe is 39 % busy, the rest
 // is the table phase, which one block per SM cannot overlap with the sums.
 template <int MG>
 __global__ void __launch_bounds__(kThreads) k_sk_noalloc_partial(const double *__restrict__ pos,
