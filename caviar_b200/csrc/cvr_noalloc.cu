@@ -128,7 +128,7 @@ __global__ void __launch_bounds__(kThreads) k_sk_noalloc_partial(const double *_
       const double scale = ax == 0 ? q[s0 + at] : 1.0;
       const double2 e1 = phase(u, 1);
       // m = 0: 1, and NaN where u is not finite (every S(k) is NaN then)
-      double2 v = m4 ? phase(u, m4) : make_double2(1.0 + 0.0 * u, 0.0);
+      double2 v = m4 ? phase(u, m4) : make_double2(isfinite(u) ? 1.0 : u - u, 0.0);
       double2 *out = tab + at * row + ax * kp + m4;
       const int len = min(4, kp - m4);
       for (int m = 0; m < len; ++m) {
